@@ -78,8 +78,10 @@ typedef struct {
                                     V-cycle on the assembled FP32 K_ff, the CG operator
                                     on its double-float values); 1 (default) level 0 of
                                     the FP32 V-cycle matrix-free (element-by-element
-                                    from K_e^0 and the cell scales), the CG operator
-                                    assembled double-float; 2 (3-D) also the CG operator
+                                    from K_e^0 and the cell scales), the CG operator in
+                                    double-float arithmetic, matrix-free too on 3-D grids
+                                    from 20,000 nodes whose K_e^0 has the box cell's
+                                    symmetry, else assembled; 2 (3-D) also the CG operator
                                     matrix-free: FP32 element products inside CG, with
                                     the true residual of every restart taken by an FP64
                                     matrix-free product (iterative refinement) */

@@ -8,6 +8,7 @@
 #include "galerkin.cuh"
 #include "kernels.cuh"
 #include "mfree.cuh"
+#include "mfree_parity.cuh"
 #include "mfree_tc.cuh"
 #include "nbspmv.cuh"
 
@@ -219,6 +220,19 @@ struct V<float> {
   static const float* cheb(Level& l) { return l.cheb32.p; }
 };
 
+// Level-0 vectors between node order and component planes, converting.
+template <class A, class B>
+void to_planes(const A* a, B* b, i64 nodes, cudaStream_t s) {
+  k_to_planes<A, B><<<grid_for(nodes, 256, 4096), 256, 0, s>>>(a, b, nodes);
+  SIMP_CHECK_LAUNCH();
+}
+
+template <class A, class B>
+void from_planes(const A* a, B* b, i64 nodes, cudaStream_t s) {
+  k_from_planes<A, B><<<grid_for(nodes, 256, 4096), 256, 0, s>>>(a, b, nodes);
+  SIMP_CHECK_LAUNCH();
+}
+
 template <class A, class B>
 void convert(const A* a, B* b, i64 n, cudaStream_t s) {
   k_convert<A, B><<<grid_for(n, 256, 4096), 256, 0, s>>>(a, b, n);
@@ -270,17 +284,92 @@ void mf3_tc(const MfOp& mf, const MfArgs& a, const KeF32& ke, cudaStream_t s) {
   SIMP_CHECK_LAUNCH();
 }
 
-// The tiled matrix-free kernel in the variant the tuner chose for the mode
-// (mf.tile[MODE]: shape kMfTileShape[tile % 5], float4 halo for tile >= 5;
-// every variant gives the same values), or the
-// tensor-core kernel (mf.tensor).
+// Launch of the parity kernel: the chunking of the z march that takes the
+// fewest block steps, waves x (layers + 2) -- a block's march costs its layers
+// and about two more to fill and drain (97x49x49: one wave of 5 layers 12.8
+// us, 4 layers in 1.2 waves 14.9, 8 layers in 0.6 waves 14.9).  Every
+// chunking gives the same values.
+template <class K>
+dim3 par_grid(const MfOp& mf, int rows, K kernel, int* layers) {
+  static std::mutex mu;
+  static std::unordered_map<const void*, int> resident;  // blocks the GPU holds, per kernel
+  const void* key = reinterpret_cast<const void*>(kernel);
+  int slots = 0;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    int& r = resident[key];
+    if (r == 0) {
+      int dev = 0, sms = 0, per_sm = 0;
+      SIMP_CUDA(cudaGetDevice(&dev));
+      SIMP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      SIMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * (rows + 2), 0));
+      r = std::max(1, sms * per_sm);
+    }
+    slots = r;
+  }
+  const i64 nnz = mf.nz + 1;
+  const dim3 xy((mf.nnx + kParCols - 1) / kParCols, (mf.nny + rows - 1) / rows);
+  const i64 columns = static_cast<i64>(xy.x) * xy.y;
+  i64 best = nnz, steps = std::numeric_limits<i64>::max();
+  for (i64 l = 1; l <= nnz; ++l) {
+    const i64 blocks = columns * ((nnz + l - 1) / l);
+    const i64 s = (blocks + slots - 1) / slots * (l + 2);
+    if (s < steps) {
+      steps = s;
+      best = l;
+    }
+  }
+  *layers = static_cast<int>(best);
+  return dim3(xy.x, xy.y, static_cast<unsigned>((nnz + best - 1) / best));
+}
+
 template <int MODE>
-void mf3(const MfOp& mf, const MfArgs& a, cudaStream_t s) {
+void mf3_par(const MfOp& mf, const MfArgs& a, cudaStream_t s) {
+  KePar32 ke{};
+  for (int l = 0; l < 8; ++l)
+    for (int r = 0; r < 3; ++r)
+      for (int c = 0; c < 3; ++c) ke.k[l][r][c] = static_cast<float>(mf.kpar[l][r][c]);
+  int layers = 0;
+  const dim3 grid = par_grid(mf, kParRows, k_mf3_par<MODE, ParF32, kParRows>, &layers);
+  k_mf3_par<MODE, ParF32, kParRows><<<grid, 32 * (kParRows + 2), 0, s>>>(mf_view(mf), a, ke, layers);
+  SIMP_CHECK_LAUNCH();
+}
+
+// y = A x or y = b - A x in double-float arithmetic (x in (hi, lo) pairs).
+template <int MODE>
+void mf3_df(const MfOp& mf, const float2* x, double* y, const double* b, cudaStream_t s) {
+  KeParDf ke{};
+  for (int l = 0; l < 8; ++l)
+    for (int r = 0; r < 3; ++r)
+      for (int c = 0; c < 3; ++c) {
+        ke.k[l][r][c].x = static_cast<float>(mf.kpar[l][r][c]);
+        ke.k[l][r][c].y = static_cast<float>(mf.kpar[l][r][c] - static_cast<double>(ke.k[l][r][c].x));
+      }
+  int layers = 0;
+  const dim3 grid = par_grid(mf, kParRowsDf, k_mf3_par<MODE, ParDf, kParRowsDf>, &layers);
+  const MfArgs64 a{x, y, b, mf.scale2};
+  k_mf3_par<MODE, ParDf, kParRowsDf><<<grid, 32 * (kParRowsDf + 2), 0, s>>>(mf_view(mf), a, ke, layers);
+  SIMP_CHECK_LAUNCH();
+}
+
+// The matrix-free kernel: in the parity basis (mf.planes) or the tiled direct
+// product, in the variant the tuner chose for the mode (mf.tile[MODE]), or
+// the tensor-core kernel (mf.tensor).
+template <int MODE>
+void mf3(const MfOp& mf, const MfArgs& args, cudaStream_t s) {
+  MfArgs a = args;
+  a.nodes = mf.free_nodes;
   KeF32 ke;
   std::copy(mf.ke_host, mf.ke_host + 24 * 24, ke.k);
   if (mf.tensor) {
     mf3_tc<MODE>(mf, a, ke, s);
     return;
+  }
+  if constexpr (MODE != 1 && MODE != 8) {  // (those read and write vectors in node order)
+    if (mf.planes) {
+      mf3_par<MODE>(mf, a, s);
+      return;
+    }
   }
   static_assert(kMfTiles == 10, "tile table");
   const int tile = mf.tile[MODE];
@@ -377,13 +466,21 @@ void mf_restrict(const MfOp& mf, const Level& lv, const float* x, const float* b
   c.coef = lv.omega32.p;
   mf3<7>(mf, c, s);
   const i64 th = static_cast<i64>(lv.naggs) * 32;
-  k_phat_restrict<6><<<grid_for(th, 256), 256, 0, s>>>(lv.naggs, lv.d_members_ptr.p, lv.d_members.p,
-                                                         lv.phat_ptr.p, lv.phat32.p, r, bc);
+  auto restrict_to = [&](auto kernel) {
+    kernel<<<grid_for(th, 256), 256, 0, s>>>(lv.naggs, lv.nnodes, lv.d_members_ptr.p, lv.d_members.p,
+                                             lv.phat_ptr.p, lv.phat32.p, r, bc);
+  };
+  if (mf.planes) restrict_to(k_phat_restrict<6, true>);
+  else restrict_to(k_phat_restrict<6, false>);
   SIMP_CHECK_LAUNCH();
 }
 
 void mf_prolong(const MfOp& mf, const Level& lv, const float* xc, float* t, float* x, cudaStream_t s) {
-  k_phat_prolong<6><<<grid_for(lv.n, 256), 256, 0, s>>>(lv.n, lv.d_agg.p, lv.phat_ptr.p, lv.phat32.p, xc, t);
+  auto prolong = [&](auto kernel) {
+    kernel<<<grid_for(lv.n, 256), 256, 0, s>>>(lv.n, lv.d_agg.p, lv.phat_ptr.p, lv.phat32.p, xc, t);
+  };
+  if (mf.planes) prolong(k_phat_prolong<6, true>);
+  else prolong(k_phat_prolong<6, false>);
   SIMP_CHECK_LAUNCH();
   MfArgs a{};
   a.x = t;
@@ -571,6 +668,11 @@ void GpuAmg::op0(SolveWork& w, const double* x, double* y, const double* rhs, bo
     k_split_pairs<<<grid_for(l0.n, 256, 8192), 256, 0, stream>>>(l0.n, x, xsplit);
     SIMP_CHECK_LAUNCH();
   }
+  if (par_cg()) {
+    if (rhs) mf3_df<1>(mf, xsplit, y, rhs, stream);
+    else mf3_df<0>(mf, xsplit, y, nullptr, stream);
+    return;
+  }
   df_apply(xsplit, y, rhs, stream);
 }
 
@@ -606,7 +708,7 @@ void GpuAmg::df_apply_unroll(const float2* xsplit, double* y, const double* rhs,
 // 8 row steps in flight per lane on y = A x (the same bits), before the
 // first CUDA graph capture of a structure.
 void GpuAmg::tune_df() {
-  if (!mixed() || mf_cg()) return;
+  if (!mixed() || mf_cg() || par_cg()) return;
   Level& l0 = *levels.front();
   const i32 n = l0.n;
   DBuf<float2> xs(static_cast<size_t>(n));
@@ -662,6 +764,12 @@ void GpuAmg::spmv0_fast(const double* x, double* y) {
   }
   const i32 n = l0.n;
   LevelWork& v = work(0).lv.front();  // the cycle's level-0 vectors are free between solves
+  if (mf.planes) {
+    to_planes(x, v.d32.p, l0.nnodes, stream);
+    mf_apply(mf, l0.nnodes, v.d32.p, v.e32.p, stream);
+    from_planes(v.e32.p, y, l0.nnodes, stream);
+    return;
+  }
   convert(x, v.d32.p, n, stream);
   if (mf.enabled) {
     mf_apply(mf, l0.nnodes, v.d32.p, v.e32.p, stream);
@@ -720,6 +828,11 @@ void GpuAmg::time_operator(int reps, double* ms, double* bytes) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   *ms = t / std::max(reps, 1);
+  if (par_cg()) {  // x and y, a scale per cell, a free-node index per grid node
+    *bytes = 2.0 * static_cast<double>(n) * 8.0 + 8.0 * mf.nx * static_cast<double>(mf.ny) * mf.nz +
+             4.0 * mf.nnx * static_cast<double>(mf.nny) * (mf.nz + 1);
+    return;
+  }
   // values, then the index data the kernel reads: one slot record per block
   // with the column-free decode (else a column per value), row pointers,
   // row -> node map and node pointers; then x once and y once
@@ -732,6 +845,10 @@ void GpuAmg::time_operator(int reps, double* ms, double* bytes) {
 void GpuAmg::refresh_level0_fp32() {
   Level& l0 = *levels.front();
   l0.a.v32.alloc(static_cast<size_t>(l0.a.nnz));
+  if (par_cg()) {
+    convert(l0.a.v64.p, l0.a.v32.p, l0.a.nnz, stream);
+    return;
+  }
   l0.a.v2.alloc(static_cast<size_t>(l0.a.nnz));
   k_split_values_pairs<<<grid_for(l0.a.nnz, 256, 8192), 256, 0, stream>>>(l0.a.nnz, l0.a.v64.p, l0.a.v32.p,
                                                                            l0.a.v2.p);
@@ -765,11 +882,9 @@ void GpuAmg::lanczos(size_t l, int m, double* ab) {
   T* w = bufs[2].p;
   T* s = bufs[3].p;
   T* tmp = bufs[4].p;
-  if constexpr (std::is_same<T, double>::value)
-    SIMP_CUDA(cudaMemcpyAsync(v, lv.lz_start.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
-  else
-    convert(lv.lz_start.p, v, n, stream);
-  k_lanczos_start<T><<<grid_for(n, 256), 256, 0, stream>>>(v, scal.p + 1, lv.dinv64.p, s, tmp, n);
+  const i64 planes = l == 0 && mf.planes ? lv.nnodes : 0;
+  k_lanczos_start<T><<<grid_for(n, 256), 256, 0, stream>>>(lv.lz_start.p, v, scal.p + 1, lv.dinv64.p, s, tmp, n,
+                                                          planes);
   SIMP_CHECK_LAUNCH();
   for (int j = 0; j < m; ++j) {
     if constexpr (std::is_same<T, float>::value) {
@@ -816,7 +931,7 @@ void GpuAmg::numeric_level(size_t l) {
   SIMP_CHECK_LAUNCH();
   // the diagonal's status is read with the Lanczos coefficients below (one
   // host round trip per level); a bad diagonal only makes them garbage
-  if (mixed()) {
+  if (mixed() && l > 0) {  // (level 0's copy follows when its vectors' order is known)
     lv.dinv32.alloc(n);
     convert(lv.dinv64.p, lv.dinv32.p, n, stream);
   }
@@ -1255,6 +1370,7 @@ void GpuAmg::setup(bool structure_changed) {
     if (mf.tensor && mf.tc_layers <= 0) mf.tc_layers = tc_layers_of(mf, 0);
   }
   if (!reuse) {
+    mf.planes = false;
     while (levels.size() > 1) levels.pop_back();
     Level& l0 = *levels.front();
     l0.agg.clear();
@@ -1283,6 +1399,15 @@ void GpuAmg::setup(bool structure_changed) {
   }
   levels.resize(l + 1);
   for (size_t k = 0; k < levels.size(); ++k) make_ops(k);
+  if (mixed()) {
+    Level& l0 = *levels.front();
+    mf.free_nodes = l0.nnodes;
+    mf.planes = mf.enabled && mf.dim == 3 && mf.parity && !mf.tensor && opt.mf_transfer && levels.size() > 1 &&
+                l0.mf_transfer && mf.grid_nodes() >= kParCycleNodes;
+    l0.dinv32.alloc(static_cast<size_t>(l0.n));
+    if (mf.planes) to_planes(l0.dinv64.p, l0.dinv32.p, l0.nnodes, stream);
+    else convert(l0.dinv64.p, l0.dinv32.p, l0.n, stream);
+  }
   coarse_factorize();
   ensure(main_);
   for (auto& w : extra_) ensure(*w);
@@ -1358,6 +1483,11 @@ void GpuAmg::tune_level0() {
                               },
                               stream, 0, 5);
   };
+  if (mf.planes) {  // the parity kernel's launch follows a rule (par_grid)
+    if (mf_cg()) tune_mode(8, [&](const MfOp& m) { mf3<8>(m, a, stream); });
+    SIMP_CUDA(cudaStreamSynchronize(stream));
+    return;
+  }
   tune_mode(0, [&](const MfOp& m) { mf3<0>(m, a, stream); });
   tune_mode(1, [&](const MfOp& m) { mf3<1>(m, a, stream); });
   tune_mode(3, [&](const MfOp& m) { mf3<3>(m, a, stream); });
@@ -1465,7 +1595,11 @@ void GpuAmg::apply(SolveWork& w, const double* r, double* z) {
   if (!ready_) throw Error(kBadInput, "multigrid: apply() called before setup()");
   Level& f = *levels.front();
   LevelWork& v = w.lv.front();
-  if (mixed()) {
+  if (mf.planes) {
+    to_planes(r, v.b32.p, f.nnodes, w.stream);
+    cycle<float>(w, 0);
+    from_planes(v.x32.p, z, f.nnodes, w.stream);
+  } else if (mixed()) {
     convert(r, v.b32.p, f.n, w.stream);
     cycle<float>(w, 0);
     convert(v.x32.p, z, f.n, w.stream);
@@ -1569,7 +1703,7 @@ GpuAmg::PcgResult GpuAmg::pcg(SolveWork& w, const double* b, double* x_out, doub
   auto apply = [&](const double* r, double* z) { this->apply(w, r, z); };
   // mixed: the direction update also writes p's double-float split (or,
   // with the matrix-free CG operator, its FP32 copy)
-  float2* psplit = mixed() && !mf_cg() ? w.xsplit.p : nullptr;
+  float2* psplit = psplit_of(w);
   if (mf_cg()) w.p32.alloc(static_cast<size_t>(n));
   const bool p_copy = psplit != nullptr || mf_cg();
   bool p_split = false;
@@ -1765,7 +1899,7 @@ struct TogetherGraph {
     std::vector<char> fused(n, 0);
     for (size_t i = 0; i < n; ++i) {
       GpuAmg* a = members[i].first;
-      if (!a->mixed() || a->mf_cg()) continue;
+      if (!a->mixed() || a->mf_cg() || a->par_cg()) continue;
       if (static_cast<double>(a->levels.front()->a.nnz) * 8.0 < kFuseBytes) continue;
       bool placed = false;
       for (auto& grp : groups)

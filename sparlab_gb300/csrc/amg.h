@@ -132,6 +132,16 @@ struct Level {
 
 // Matrix-free level-0 operator of a structured grid (see mfree.cuh), used
 // by the FP32 V-cycle and the mixed-precision CG operator when enabled.
+// Grid nodes from which the double-float CG operator and the FP32 cycle run in
+// the parity basis.  Below them the march along z is too short to hide its
+// steps' latency and K_ff's pairs sit in L2: the CG product takes 10.4 us
+// against 6.4 at 32x16x8 cells (5 k nodes), about the same at 40x20x15, 16.5
+// against 36.6 at 61x37x29 (71 k); a cycle product takes 8.7 against 6.7 us at
+// 71 k nodes, the evaluation the same time either way at 96x48x24 (119 k), and
+// 12.8 against 16.9 us at 96x48x48 (233 k).
+constexpr i64 kParCgNodes = 20000;
+constexpr i64 kParCycleNodes = 150000;
+
 struct MfOp {
   bool enabled = false;
   int dim = 3;
@@ -144,8 +154,18 @@ struct MfOp {
   // variant of the tiled 3-D kernel per mode (0..8): shape
   // kMfTileShape[tile % 5], float4 halo if >= 5 (tuned per mode)
   int tile[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const float2* scale2 = nullptr;   // s_e as (hi, lo) pairs (the double-float parity product)
   const double* scale64 = nullptr;  // s_e, FP64 (the matrix-free CG operator's true residuals)
   double ke64_host[24 * 24] = {};   // K_e^0, FP64
+  // 3-D: K_e^0 has the box cell's symmetry, and its parity blocks
+  // (mfree_parity.cuh)
+  bool parity = false;
+  double kpar[8][3][3] = {};
+  // the FP32 cycle's level-0 products run in the parity basis, with level
+  // 0's FP32 vectors in component planes (set by the setup)
+  bool planes = false;
+  i32 free_nodes = 0;
+  i64 grid_nodes() const { return static_cast<i64>(nnx) * nny * (nz + 1); }
   bool tensor = false;     // 3-D: the tensor-core kernel (mfree_tc.cuh) instead of the tiled FMA kernel
   int tc_layers = 0;       // node layers per CTA of the tensor-core kernel (tuned; 0: all)
   int* status = nullptr;   // device word the tensor-core kernel sets when a wait runs out
@@ -217,6 +237,12 @@ class GpuAmg {
   bool mixed() const { return opt.precision == 1; }
   // the CG operator is the FP32 matrix-free product (matrix_free = 2, 3-D)
   bool mf_cg() const { return mixed() && opt.matrix_free >= 2 && mf.enabled && mf.dim == 3; }
+  // the CG operator and the true residuals are matrix-free double-float
+  // products (mfree_parity.cuh): no (hi, lo) pairs of K_ff are kept
+  bool par_cg() const {
+    return mixed() && opt.matrix_free == 1 && mf.enabled && mf.dim == 3 && mf.parity &&
+           mf.grid_nodes() >= kParCgNodes;
+  }
   // Set by an assembler that wrote level 0's FP32 values (hi in a.v32 and
   // (hi, lo) pairs in a.v2) itself; otherwise setup splits the FP64 values (mixed
   // mode).  In mixed mode the CG operator reads hi/lo only, so an assembler

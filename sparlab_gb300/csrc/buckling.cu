@@ -377,12 +377,16 @@ BucklingResult solve_buckling(GpuProblem& p, const BucklingOptions& o, int load_
   p.assemble_into(p.ke_d.p, ks.p, true, l0.a.v64.p, nullptr, nullptr, s);
   const double* kval = l0.a.v64.p;
   DBuf<float> ks32;
+  DBuf<float2> ks2;
   if (p.amg.mf.enabled) {
     ks32.alloc(static_cast<size_t>(ne));
-    k_convert<double, float><<<grid_for(ne, 256), 256, 0, s>>>(ks.p, ks32.p, ne);
+    ks2.alloc(static_cast<size_t>(ne));
+    k_split_values_pairs<<<grid_for(ne, 256), 256, 0, s>>>(ne, ks.p, ks32.p, ks2.p);
     SIMP_CHECK_LAUNCH();
     amg.mf = p.amg.mf;
     amg.mf.scale = ks32.p;
+    amg.mf.scale2 = ks2.p;
+    amg.mf.scale64 = ks.p;
   }
   amg.setup(true);
   SolveWork& w0 = amg.work(0);

@@ -88,15 +88,6 @@ __device__ __forceinline__ void df_split(double v, float& hi, float& lo) {
   lo = __double2float_rn(v - static_cast<double>(hi));
 }
 
-__global__ void k_split_values(i64 n, const double* __restrict__ v, float* __restrict__ hi, float* __restrict__ lo) {
-  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-    float h, l;
-    df_split(v[i], h, l);
-    if (hi) hi[i] = h;
-    lo[i] = l;
-  }
-}
-
 // hi = float(v) and the interleaved (hi, lo) pairs of the double-float operator
 __global__ void k_split_values_pairs(i64 n, const double* __restrict__ v, float* __restrict__ hi,
                                      float2* __restrict__ pair) {
@@ -148,6 +139,21 @@ template <class A, class B>
 __global__ void k_convert(const A* __restrict__ a, B* __restrict__ b, i64 n) {
   for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
     b[i] = static_cast<B>(a[i]);
+}
+
+// three unknowns a node: node order (3 I + k) to component planes (k nodes + I) and back
+template <class A, class B>
+__global__ void k_to_planes(const A* __restrict__ a, B* __restrict__ b, i64 nodes) {
+  for (i64 I = blockIdx.x * (i64)blockDim.x + threadIdx.x; I < nodes; I += (i64)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) b[k * nodes + I] = static_cast<B>(a[3 * I + k]);
+}
+
+template <class A, class B>
+__global__ void k_from_planes(const A* __restrict__ a, B* __restrict__ b, i64 nodes) {
+  for (i64 I = blockIdx.x * (i64)blockDim.x + threadIdx.x; I < nodes; I += (i64)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) b[3 * I + k] = static_cast<B>(a[k * nodes + I]);
 }
 
 // ---------------------------------------------------------------------------
@@ -342,18 +348,20 @@ __global__ void k_lanczos_shift(T* __restrict__ v, T* __restrict__ vp, const T* 
   }
 }
 
-// v = v / nrm ; tmp = s .* v ; s = sqrt(dinv)
+// v = start / nrm ; tmp = s .* v ; s = sqrt(dinv).  planes > 0: v, s and tmp in
+// component planes of that many nodes (three unknowns a node).
 template <class T>
-__global__ void k_lanczos_start(T* __restrict__ v, const double* __restrict__ nrm,
-                                const double* __restrict__ dinv, T* __restrict__ s,
-                                T* __restrict__ tmp, i64 n) {
+__global__ void k_lanczos_start(const double* __restrict__ start, T* __restrict__ v,
+                                const double* __restrict__ nrm, const double* __restrict__ dinv,
+                                T* __restrict__ s, T* __restrict__ tmp, i64 n, i64 planes) {
   const double inv = *nrm;
   for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
+    const i64 o = planes > 0 ? (i % 3) * planes + i / 3 : i;
     const double si = sqrt(dinv[i]);
-    s[i] = static_cast<T>(si);
-    const double vi = todbl(v[i]) / inv;
-    v[i] = static_cast<T>(vi);
-    tmp[i] = static_cast<T>(todbl(static_cast<T>(si)) * todbl(static_cast<T>(vi)));
+    s[o] = static_cast<T>(si);
+    const double vi = todbl(static_cast<T>(start[i])) / inv;
+    v[o] = static_cast<T>(vi);
+    tmp[o] = static_cast<T>(todbl(static_cast<T>(si)) * todbl(static_cast<T>(vi)));
   }
 }
 

@@ -180,7 +180,20 @@ struct MfArgs {
   const float* coef;  // mode 3: (c1, c2); mode 4: 1 / theta; mode 5/7: w (device memory)
   int add_d;
   double* y64;        // mode 8: output
+  i32 nodes;          // free nodes (stride of the component planes)
 };
+
+// Unknown (node I, component k) of a level-0 vector: node by node, or (SOA)
+// in component planes, as a plane's base (the same for every thread) and a
+// 32-bit byte offset shared by all vectors and planes.
+template <bool SOA, class T>
+__device__ __forceinline__ T* mf_place(const MfArgs& a, T* v, i32 I, int k) {
+  if constexpr (SOA)
+    return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(v + static_cast<i64>(k) * a.nodes) +
+                                static_cast<uint32_t>(I) * static_cast<uint32_t>(sizeof(T)));
+  else
+    return v + 3 * static_cast<i64>(I) + k;
+}
 
 // The epilogue of a node's product o = (A x)_I (3 components) in each mode,
 // in two parts: the node's operand loads (mf_node_load: right-hand side,
@@ -192,50 +205,50 @@ struct MfNodeIn {
   float b[3], dinv[3], xs[3];
 };
 
-template <int MODE>
+template <int MODE, bool SOA = false>
 __device__ __forceinline__ void mf_node_load(const MfArgs& a, i32 I, MfNodeIn& in) {
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const i64 row = static_cast<i64>(I) * 3 + k;
-    if (MODE == 1 || MODE == 3 || MODE == 4 || MODE == 6 || MODE == 7) in.b[k] = a.b[row];
-    if (MODE == 3 || MODE == 4 || MODE == 5 || MODE == 6) in.dinv[k] = a.dinv[row];
-    if (MODE == 3 || MODE == 5) in.xs[k] = a.xs[row];
+    auto at = [&](auto* v) -> auto& { return *mf_place<SOA>(a, v, I, k); };
+    if (MODE == 1 || MODE == 3 || MODE == 4 || MODE == 6 || MODE == 7) in.b[k] = at(a.b);
+    if (MODE == 3 || MODE == 4 || MODE == 5 || MODE == 6) in.dinv[k] = at(a.dinv);
+    if (MODE == 3 || MODE == 5) in.xs[k] = at(a.xs);
   }
 }
 
-template <int MODE>
+template <int MODE, bool SOA = false>
 __device__ __forceinline__ void mf_node_store(const MfArgs& a, i32 I, const float (&o)[3], const float (&self)[3],
                                               const MfNodeIn& in, float c0, float c1) {
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const i64 row = static_cast<i64>(I) * 3 + k;
+    auto at = [&](auto* v) -> auto& { return *mf_place<SOA>(a, v, I, k); };
     if (MODE == 0) {
-      a.y[row] = o[k];
+      at(a.y) = o[k];
     } else if (MODE == 1) {
-      a.y[row] = in.b[k] - o[k];
+      at(a.y) = in.b[k] - o[k];
     } else if (MODE == 3) {
       const float ri = in.b[k] - o[k];
-      a.r[row] = ri;
+      at(a.r) = ri;
       const float dv = self[k];
       const float di = c0 * dv + c1 * in.dinv[k] * ri;
-      a.dn[row] = di;
+      at(a.dn) = di;
       float xi = in.xs[k];
       if (a.add_d) xi = xi + dv;
-      a.xs[row] = xi + di;
+      at(a.xs) = xi + di;
     } else if (MODE == 4) {
       const float ri = in.b[k] - o[k];
-      a.r[row] = ri;
-      a.dn[row] = in.dinv[k] * ri * c0;
+      at(a.r) = ri;
+      at(a.dn) = in.dinv[k] * ri * c0;
     } else if (MODE == 5) {
-      a.xs[row] = in.xs[k] + (self[k] - c0 * (in.dinv[k] * o[k]));
+      at(a.xs) = in.xs[k] + (self[k] - c0 * (in.dinv[k] * o[k]));
     } else if (MODE == 6) {
       const float ri = in.b[k] - o[k];
-      a.y[row] = ri;
-      a.dn[row] = in.dinv[k] * ri;
+      at(a.y) = ri;
+      at(a.dn) = in.dinv[k] * ri;
     } else if (MODE == 8) {
-      a.y64[row] = static_cast<double>(o[k]);
+      a.y64[3 * static_cast<i64>(I) + k] = static_cast<double>(o[k]);
     } else {
-      a.y[row] = in.b[k] - c0 * o[k];
+      at(a.y) = in.b[k] - c0 * o[k];
     }
   }
 }
@@ -486,10 +499,10 @@ __global__ void __launch_bounds__(kTX* kTY* kTZ) k_mf3_tile64(MfView m, const do
 }
 
 // The tentative prolongator P^ of level 0 (3 unknowns per node, B1 per
-// aggregate; aggregate g owns coarse unknowns g B1 .. g B1 + B1 - 1; the row
+// aggregate; SOA: t in component planes; aggregate g owns coarse unknowns g B1 .. g B1 + B1 - 1; the row
 // of fine unknown i is phat[phat_ptr[i] ...], B1 values, empty for a node in
 // no aggregate).  t = P^ x_c, one thread per fine unknown.
-template <int B1>
+template <int B1, bool SOA>
 __global__ void __launch_bounds__(256) k_phat_prolong(i32 n, const i32* __restrict__ agg,
                                                       const i32* __restrict__ phat_ptr,
                                                       const float* __restrict__ phat, const float* __restrict__ xc,
@@ -504,14 +517,14 @@ __global__ void __launch_bounds__(256) k_phat_prolong(i32 n, const i32* __restri
 #pragma unroll
     for (int j = 0; j < B1; ++j) s = fmaf(ph[j], xg[j], s);
   }
-  t[i] = s;
+  t[SOA ? static_cast<i64>(i % 3) * (n / 3) + i / 3 : i] = s;
 }
 
 // b_c = P^T t: one warp per aggregate; lane q takes the aggregate's member
 // unknowns q, q + 32, ... (members ascending, 3 unknowns each) into B1 partial
 // sums, reduced across the warp in a fixed butterfly order.
-template <int B1>
-__global__ void __launch_bounds__(256) k_phat_restrict(i32 naggs, const i32* __restrict__ mptr,
+template <int B1, bool SOA>
+__global__ void __launch_bounds__(256) k_phat_restrict(i32 naggs, i64 nodes, const i32* __restrict__ mptr,
                                                        const i32* __restrict__ members,
                                                        const i32* __restrict__ phat_ptr,
                                                        const float* __restrict__ phat, const float* __restrict__ t,
@@ -525,7 +538,7 @@ __global__ void __launch_bounds__(256) k_phat_restrict(i32 naggs, const i32* __r
   for (int j = 0; j < B1; ++j) acc[j] = 0.0f;
   for (i32 q = lane; q < cnt; q += 32) {
     const i32 i = 3 * members[q0 + q / 3] + q % 3;
-    const float ti = t[i];
+    const float ti = t[SOA ? (i % 3) * nodes + i / 3 : i];
     const float* ph = phat + phat_ptr[i];
 #pragma unroll
     for (int j = 0; j < B1; ++j) acc[j] = fmaf(ph[j], ti, acc[j]);

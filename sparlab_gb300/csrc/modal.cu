@@ -380,12 +380,16 @@ ModalResult solve_modal(GpuProblem& p, const ModalOptions& o, const double* ksca
     // operator is the matrix-free K (FP32), as in the optimisation's solver;
     // only without a shift, where A = K
     DBuf<float> ks32;
+    DBuf<float2> ks2;
     if (p.amg.mf.enabled && sigma == 0.0) {
       ks32.alloc(static_cast<size_t>(ne));
-      k_convert<double, float><<<grid_for(ne, 256), 256, 0, s>>>(ks.p, ks32.p, ne);
+      ks2.alloc(static_cast<size_t>(ne));
+      k_split_values_pairs<<<grid_for(ne, 256), 256, 0, s>>>(ne, ks.p, ks32.p, ks2.p);
       SIMP_CHECK_LAUNCH();
       amg.mf = p.amg.mf;
       amg.mf.scale = ks32.p;
+      amg.mf.scale2 = ks2.p;
+      amg.mf.scale64 = ks.p;
     }
     amg.setup(true);
     const std::vector<SolveWork*> works = workspaces(amg, std::max(1, std::min(q, o.concurrent_solves)));

@@ -3,6 +3,7 @@
 #include "problem.h"
 #include "surrogate_net.h"
 #include "topopt.cuh"
+#include "mfree_parity.cuh"
 
 #include <algorithm>
 #include <array>
@@ -257,7 +258,6 @@ void GpuProblem::build() {
     if (amg.mixed() && all_or_nothing && amg.opt.matrix_free >= 1) {
       std::vector<float> k32(d.ke.begin(), d.ke.end());
       ke32.upload(k32);
-      sf32.alloc(static_cast<size_t>(ne));
       nindex.upload(node_index);
       MfOp& mf = amg.mf;
       mf.enabled = true;
@@ -272,7 +272,7 @@ void GpuProblem::build() {
       mf.ke = ke32.p;
       std::copy(k32.begin(), k32.end(), mf.ke_host);
       std::copy(d.ke.begin(), d.ke.end(), mf.ke64_host);
-      mf.scale = sf32.p;
+      mf.parity = dim == 3 && parity_blocks(d.ke.data(), mf.kpar);
     }
   }
   std::vector<uint8_t> uc(ucomp_h.begin(), ucomp_h.end());
@@ -285,6 +285,12 @@ void GpuProblem::build() {
   xnew.alloc(ne_s);
   rho.alloc(ne_s);
   sf.alloc(ne_s);
+  if (amg.mixed()) {
+    sf32.alloc(ne_s);
+    sf2.alloc(ne_s);
+    amg.mf.scale = sf32.p;
+    amg.mf.scale2 = sf2.p;
+  }
   amg.mf.scale64 = sf.p;  // the FP64 SIMP factors (matrix-free CG operator)
   df.alloc(ne_s);
   dc_dphys.alloc(ne_s);
@@ -459,7 +465,7 @@ void GpuProblem::assemble_into(const double* elem, const double* scale, bool exa
   raise_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   kernel<<<blocks, assemble_threads(d.dim), smem, stream>>>(grid_of(d), l0.nnodes, l0.d_first.p, gnode.p, cmask.p,
                                                             nmask.p, l0.d_apat.view(), l0.a.ptr.p, elem, scale,
-                                                            nullptr, nullptr, v64, hi, pair);
+                                                            nullptr, v64, hi, pair);
   SIMP_CHECK_LAUNCH();
 }
 
@@ -470,34 +476,30 @@ void GpuProblem::assemble(const double* scale, bool exact) {
   const unsigned blocks = static_cast<unsigned>((l0.nnodes + kAsmTile - 1) / kAsmTile);
   const size_t smem = assemble_smem(d.dim);
   const int threads = assemble_threads(d.dim);
-  auto launch = [&](auto kernel, const float* sh, const float* sl, double* v64, float* hi, float2* pair) {
+  auto launch = [&](auto kernel, const float2* scale2, double* v64, float* hi, float2* pair) {
     raise_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     kernel<<<blocks, threads, smem, amg.stream>>>(g, l0.nnodes, l0.d_first.p, gnode.p, cmask.p, nmask.p,
-                                                  l0.d_apat.view(), l0.a.ptr.p, ke_d.p, scale, sh, sl, v64, hi,
+                                                  l0.d_apat.view(), l0.a.ptr.p, ke_d.p, scale, scale2, v64, hi,
                                                   pair);
     SIMP_CHECK_LAUNCH();
   };
   if (!amg.mixed()) {
-    if (exact) launch(k_assemble_tiles<true, false>, nullptr, nullptr, l0.a.v64.p, nullptr, nullptr);
-    else launch(k_assemble_tiles<false, false>, nullptr, nullptr, l0.a.v64.p, nullptr, nullptr);
+    if (exact) launch(k_assemble_tiles<true, false>, nullptr, l0.a.v64.p, nullptr, nullptr);
+    else launch(k_assemble_tiles<false, false>, nullptr, l0.a.v64.p, nullptr, nullptr);
     return;
   }
   // mixed: the double-float split (hi = the FP32 values of the preconditioner,
-  // hi + lo = the CG operator); FP64 values only for the structure-defining
-  // exact assembly
+  // hi + lo = the assembled CG operator, not kept where it is matrix-free);
+  // FP64 values only for the structure-defining exact assembly
   l0.a.v32.alloc(static_cast<size_t>(l0.a.nnz));
-  l0.a.v2.alloc(static_cast<size_t>(l0.a.nnz));
+  if (!amg.par_cg()) l0.a.v2.alloc(static_cast<size_t>(l0.a.nnz));
   if (exact) {
-    launch(k_assemble_tiles<true, false>, nullptr, nullptr, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
+    launch(k_assemble_tiles<true, false>, nullptr, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
   } else if (!amg.opt.reuse) {
     // every setup rebuilds the hierarchy from FP64 values
-    launch(k_assemble_tiles<false, false>, nullptr, nullptr, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
+    launch(k_assemble_tiles<false, false>, nullptr, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
   } else {
-    scale_hi.alloc(static_cast<size_t>(ne));
-    scale_lo.alloc(static_cast<size_t>(ne));
-    k_split_values<<<grid_for(ne, 256, 8192), 256, 0, amg.stream>>>(ne, scale, scale_hi.p, scale_lo.p);
-    SIMP_CHECK_LAUNCH();
-    launch(k_assemble_tiles<false, true>, scale_hi.p, scale_lo.p, nullptr, l0.a.v32.p, l0.a.v2.p);
+    launch(k_assemble_tiles<false, true>, sf2.p, nullptr, l0.a.v32.p, l0.a.v2.p);
   }
   amg.level0_fp32_fresh = true;
 }
@@ -540,8 +542,8 @@ void GpuProblem::evaluate_prepare() {
   }
   k_simp<<<grid_for(ne, 256), 256, 0, s>>>(ne, rho.p, d.penalty, d.emin, sf.p, df.p);
   SIMP_CHECK_LAUNCH();
-  if (amg.mf.enabled) {
-    k_convert<double, float><<<grid_for(ne, 256), 256, 0, s>>>(sf.p, sf32.p, ne);
+  if (amg.mixed()) {
+    k_split_values_pairs<<<grid_for(ne, 256), 256, 0, s>>>(ne, sf.p, sf32.p, sf2.p);
     SIMP_CHECK_LAUNCH();
   }
   if (d.warm == 3 && surrogate) {

@@ -120,7 +120,7 @@ class GpuProblem {
   DBuf<double> oc_g, oc_lo, oc_hi;  // OC candidate factors of the current update
   // matrix-free level-0 operator (mixed precision, fully free / clamped nodes)
   DBuf<float> ke32, sf32;
-  DBuf<float> scale_hi, scale_lo;  // double-float split of the stiffness factors (mixed assembly)
+  DBuf<float2> sf2;  // the stiffness factors as (hi, lo) pairs (mixed precision)
   DBuf<i32> nindex;
   void* stencil_d = nullptr;
   std::vector<double> last_compliance;

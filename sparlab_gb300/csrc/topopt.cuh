@@ -58,7 +58,7 @@ inline size_t assemble_smem(int dim) {
 
 // Outputs: val64 (FP64 values), hi (FP32) and pair (the double-float split
 // (hi, lo), interleaved), each optional.  DF: the sums themselves run in double-float arithmetic on
-// the FP32 pipes from the split scales (sh, sl) and the split element matrix
+// the FP32 pipes from the split scales (hi, lo) and the split element matrix
 // (the mixed-precision reuse assemblies, which write hi/lo only); otherwise
 // in FP64 (EXACT: rounded products and sums; else fused multiply-adds).
 template <bool EXACT, bool DF>
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(kAsmGroups3 * kAsmTile) k_assemble_tiles(
     GridView g, i32 nodes, const i32* __restrict__ first, const i32* __restrict__ gnode,
     const uint8_t* __restrict__ cmask, const uint32_t* __restrict__ nmask, NodeView a,
     const i32* __restrict__ rowptr, const double* __restrict__ ke, const double* __restrict__ scale,
-    const float* __restrict__ scale_hi, const float* __restrict__ scale_lo, double* __restrict__ val64,
+    const float2* __restrict__ scale2, double* __restrict__ val64,
     float* __restrict__ hi, float2* __restrict__ pair) {
   extern __shared__ double smem_asm[];
   const int ed = g.dim == 3 ? 24 : 8;
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kAsmGroups3 * kAsmTile) k_assemble_tiles(
           const int aI = corner_of(ix - cx, iy - cy, g.dim == 3 ? iz - cz : 0);
           const int aJ = corner_of(jx - cx, jy - cy, g.dim == 3 ? jz - cz : 0);
           if constexpr (DF) {
-            const float sh = scale_hi[c], sl = scale_lo[c];
+            const float sh = scale2[c].x, sl = scale2[c].y;
 #pragma unroll
             for (int ka = 0; ka < 3; ++ka)
 #pragma unroll
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kAsmGroups3 * kAsmTile) k_assemble_tiles(
     if constexpr (DF) {
       const float2 v = stage2[k];
       hi[base + k] = v.x;
-      pair[base + k] = v;
+      if (pair) pair[base + k] = v;
     } else {
       const double v = stage[k];
       if (val64) val64[base + k] = v;
