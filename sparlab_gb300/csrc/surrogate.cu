@@ -8,9 +8,11 @@
 #include "common.h"
 #include "conv_tc.cuh"
 #include "surrogate.h"
+#include "wgrad_tc.cuh"
 
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <sstream>
@@ -128,7 +130,8 @@ void conv_launch(const ConvSpec& s, cudaStream_t stream) {
 }
 
 // ---------------------------------------------------------------------------
-// Weight and bias gradients on the CUDA cores (FP32 accumulation):
+// Weight and bias gradients on the CUDA cores (FP32 accumulation), for the
+// channel counts that the tensor-core kernel (wgrad_tc.cuh) does not take:
 // dW_t[co][ci] = sum_v dY[v][co] X[v + o_t][ci], db[co] = sum_v dY[v][co].
 // Block (tap t, group g) sums the voxel chunks g, g + G, ... of 128 nodes in
 // a fixed order into its partial; k_wgrad_sum adds the G partials in order.
@@ -219,8 +222,58 @@ __global__ void k_wgrad_sum(int cout, int cin, int groups, const float* __restri
   }
 }
 
+// Channel counts and alignment that the tensor-core kernel takes (the
+// surrogate's own layers): 16-byte pieces of 8 channels.
+static bool wgrad_on_tensor_cores(const WgradSpec& s) {
+  auto whole = [](int c) { return c == 16 || c == 32 || c == 64; };
+  auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  return whole(s.c0) && aligned(s.x0) && (s.nseg < 2 || (whole(s.c1) && aligned(s.x1))) && whole(s.cdy) &&
+         s.cout <= s.cdy && aligned(s.dy);
+}
+
+constexpr int kWgWalkers = 152;  // CTAs over all groups: one per SM
+
+static void wgrad_tc_launch(const WgradSpec& s, float* part, cudaStream_t stream) {
+  wg::Args a{};
+  a.nx = s.nx;
+  a.ny = s.ny;
+  a.nz = s.nz;
+  a.dy = s.dy;
+  a.cdy = s.cdy;
+  a.part = part;
+  a.status = s.status;
+  a.run = static_cast<i64>(s.nx) * s.ny * s.nz <= (1 << 15) ? 2 : 4;
+  int nseg = 0, cmax = 0;
+  auto add = [&](const __nv_bfloat16* x, int c, int ci0) {
+    for (int k = 0; k < c; k += 32) {
+      wg::Segment& g = a.seg[nseg++];
+      g.x = x + k;
+      g.pitch = c;
+      g.c = std::min(32, c - k);
+      g.ci0 = ci0 + k;
+      cmax = std::max(cmax, g.c);
+    }
+  };
+  add(s.x0, s.c0, 0);
+  if (s.nseg > 1) add(s.x1, s.c1, s.c0);
+  const int cin = s.c0 + (s.nseg > 1 ? s.c1 : 0);
+  const i64 tiles = static_cast<i64>((s.nx + wg::kTX - 1) / wg::kTX) * ((s.ny + wg::kTY - 1) / wg::kTY) * s.nz;
+  const int walkers = static_cast<int>(std::max<i64>(1, std::min<i64>(tiles, kWgWalkers / (3 * nseg))));
+  const int smem = wg::smem_bytes(s.cdy, cmax);
+  raise_dynamic_smem(reinterpret_cast<const void*>(wg::k_wgrad_tc), static_cast<size_t>(smem));
+  wg::k_wgrad_tc<<<dim3(static_cast<unsigned>(walkers), static_cast<unsigned>(3 * nseg)), wg::kThreads, smem, stream>>>(a);
+  SIMP_CHECK_LAUNCH();
+  wg::k_wgrad_tc_sum<<<grid_for(27 * s.cout * cin + s.cout, 256, 1024), 256, 0, stream>>>(a, walkers, s.cout, cin, nseg,
+                                                                                         s.gw, s.gb);
+  SIMP_CHECK_LAUNCH();
+}
+
 void wgrad_launch(const WgradSpec& s, float* part, cudaStream_t stream) {
   const int cin = s.c0 + (s.nseg > 1 ? s.c1 : 0);
+  if (wgrad_on_tensor_cores(s)) {
+    wgrad_tc_launch(s, part, stream);
+    return;
+  }
   if (s.cout * cin > kWgThreads * 32) throw Error(kBadInput, "surrogate: weight block too large for the gradient kernel");
   const size_t smem = sizeof(float) * kWgChunk * (s.cout + cin);
   raise_dynamic_smem(reinterpret_cast<const void*>(k_wgrad_partial), smem);
@@ -232,7 +285,12 @@ void wgrad_launch(const WgradSpec& s, float* part, cudaStream_t stream) {
   SIMP_CHECK_LAUNCH();
 }
 
-size_t wgrad_partial_floats(int cout, int cin) { return static_cast<size_t>(28) * kWgGroups * cout * cin; }
+// floats of `part` for either kernel: the CUDA-core kernel's groups, or a slot
+// of up to 64 rows for every walker of the tensor-core kernel
+size_t wgrad_partial_floats(int cout, int cin) {
+  return std::max(static_cast<size_t>(28) * kWgGroups * cout * cin,
+                  static_cast<size_t>(kWgWalkers) * 64 * wg::part_cols(32));
+}
 
 }  // namespace sg
 }  // namespace simp
@@ -330,9 +388,12 @@ int simp_conv3d_wgrad(int32_t nx, int32_t ny, int32_t nz, int32_t nseg, const vo
     s.cout = cout;
     s.gw = gw;
     s.gb = gb;
+    DBuf<int> st(1);
+    st.zero();
+    s.status = st.p;
     DBuf<float> part(sg::wgrad_partial_floats(cout, s.c0 + s.c1));
     sg::wgrad_launch(s, part.p, 0);
-    SIMP_CUDA(cudaStreamSynchronize(0));
+    if (read_status(st.p, 0)) throw Error(kCudaError, "simp_conv3d_wgrad: a pipeline wait timed out");
   });
 }
 

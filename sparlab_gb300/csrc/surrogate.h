@@ -44,6 +44,7 @@ struct WgradSpec {
   int cout = 0;  // output channels whose gradient is formed (<= cdy)
   float* gw = nullptr;  // [27][cout][c0 + c1]
   float* gb = nullptr;  // [cout]
+  int* status = nullptr;  // device word set on a wait that ran out
 };
 
 CUtensorMap act_map(const void* base, int c, int nx, int ny, int nz);

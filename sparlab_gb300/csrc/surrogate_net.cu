@@ -506,6 +506,7 @@ void Net::wgrad(int l, const void* x0, const void* x1, const void* dy) {
   s.cout = L.cout;
   s.gw = grad.p + woff[l];
   s.gb = grad.p + boff[l];
+  s.status = status.p;
   wgrad_launch(s, wpart.p, stream);
 }
 

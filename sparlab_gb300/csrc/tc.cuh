@@ -57,9 +57,12 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 // Waits for the phase with the given parity to complete; false (and the
-// status word set) when it has not completed within kWaitNs.
+// status word set) when it has not completed within kWaitNs.  The clock is
+// read only by waits that outlast a few tries: reading the global timer costs
+// more than the short waits of a running pipeline.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status) {
-  if (mbar_try_wait(bar, parity)) return true;
+  for (int k = 0; k < 64; ++k)
+    if (mbar_try_wait(bar, parity)) return true;
   const unsigned long long t0 = global_ns();
   while (!mbar_try_wait(bar, parity)) {
     if (global_ns() - t0 > kWaitNs) {
@@ -90,6 +93,17 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 
 __device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
+
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
 }
 
 // ---- tcgen05 ----------------------------------------------------------------
