@@ -86,6 +86,26 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// The epilogue of a node's output columns c0 .. c0 + 15: bias, ReLU, store.
+__device__ __forceinline__ void conv_store(const ConvArgs& p, long long node, int c0, float (&v)[16]) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    if (p.bias) v[k] += p.bias[c0 + k];
+    if (p.relu) v[k] = fmaxf(v[k], 0.0f);
+  }
+  const int seg = (p.nout > 1 && c0 >= p.out_c[0]) ? 1 : 0;
+  const int lc = c0 - (seg ? p.out_c[0] : 0);
+  if (lc >= p.out_c[seg]) return;
+  if (p.out_f32[seg]) {
+    float* o = static_cast<float*>(p.out[seg]) + node * p.out_pitch[seg] + lc;
+    for (int k = 0; k < 16 && lc + k < p.out_c[seg]; ++k) o[k] = v[k];
+  } else {
+    uint4* o = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out[seg]) + node * p.out_pitch[seg] + lc);
+    o[0] = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+    o[1] = make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]), pack_bf16(v[14], v[15]));
+  }
+}
+
 __global__ void __launch_bounds__(kThreads) k_conv_tc(const __grid_constant__ CUtensorMap a0map,
                                                       const __grid_constant__ CUtensorMap a1map,
                                                       const __grid_constant__ CUtensorMap b0map,
@@ -98,7 +118,8 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const __grid_constant__ CU
   uint64_t* empty = full + kStages;
   uint64_t* done = empty + kStages;
   uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x) >> 5, 0);
   const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kTileY, z0 = blockIdx.z;
   const uint32_t ncols = tmem_cols(p.n);
 
@@ -138,25 +159,30 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const __grid_constant__ CU
       tc::tma_load_2d(st + abytes0 + abytes1, &b0map, 0, t * p.n, &full[s]);
       if (p.nseg > 1) tc::tma_load_2d(st + abytes0 + abytes1 + bbytes0, &b1map, p.cseg[0], t * p.n, &full[s]);
     }
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer
+  } else if (warp == 1) {
+    // MMA issuer: the whole warp runs the loop, so that descriptors stay in
+    // uniform registers; one elected lane issues
+    const bool leader = tc::elect_one();
     const uint32_t idesc = tc::idesc_bf16(128, p.n);
-    for (int t = 0; t < 27; ++t) {
+    bool ok = true;
+    for (int t = 0; t < 27 && ok; ++t) {
       const int s = t % kStages, use = t / kStages;
-      if (!tc::mbar_wait(&full[s], use & 1, p.status)) break;
+      ok = tc::mbar_wait(&full[s], use & 1, p.status);
+      if (!ok) break;
       tc::fence_after_sync();
       const uint32_t base = tc::smem_u32(smem + s * stage);
       for (int seg = 0; seg < p.nseg; ++seg) {
-        const uint32_t a_addr = base + (seg ? abytes0 : 0);
-        const uint32_t b_addr = base + abytes0 + abytes1 + (seg ? bbytes0 : 0);
         const int rb = p.cseg[seg] * 2;
-        for (int kk = 0; kk < p.cseg[seg] / 16; ++kk)
-          tc::mma_bf16(tmem, tc::smem_desc(a_addr + kk * 32, rb), tc::smem_desc(b_addr + kk * 32, rb), idesc,
-                       (t | seg | kk) != 0 ? 1u : 0u);
+        const uint64_t a = tc::smem_desc(base + (seg ? abytes0 : 0), rb);
+        const uint64_t b = tc::smem_desc(base + abytes0 + abytes1 + (seg ? bbytes0 : 0), rb);
+        if (leader)
+          for (int kk = 0; kk < p.cseg[seg] / 16; ++kk)  // 32 bytes along K
+            tc::mma_bf16(tmem, a + 2 * kk, b + 2 * kk, idesc, (t | seg | kk) != 0 ? 1u : 0u);
       }
-      tc::mma_commit(&empty[s]);
+      if (leader) tc::mma_commit(&empty[s]);
+      __syncwarp();
     }
-    tc::mma_commit(done);
+    if (leader) tc::mma_commit(done);
   }
   __syncwarp();
 
@@ -170,24 +196,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const __grid_constant__ CU
   for (int c0 = 0; c0 < p.n; c0 += 16) {
     float v[16];
     tc::tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c0), v);
-    if (!valid) continue;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      if (p.bias) v[k] += p.bias[c0 + k];
-      if (p.relu) v[k] = fmaxf(v[k], 0.0f);
-    }
-    const int seg = (p.nout > 1 && c0 >= p.out_c[0]) ? 1 : 0;
-    const int lc = c0 - (seg ? p.out_c[0] : 0);
-    if (lc >= p.out_c[seg]) continue;
-    if (p.out_f32[seg]) {
-      float* o = static_cast<float*>(p.out[seg]) + node * p.out_pitch[seg] + lc;
-      for (int k = 0; k < 16 && lc + k < p.out_c[seg]; ++k) o[k] = v[k];
-    } else {
-      uint4* o = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(p.out[seg]) + node * p.out_pitch[seg] + lc);
-      o[0] = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-      o[1] = make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]),
-                        pack_bf16(v[14], v[15]));
-    }
+    if (valid) conv_store(p, node, c0, v);
   }
   tc::fence_before_sync();
   __syncthreads();

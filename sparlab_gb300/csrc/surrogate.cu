@@ -6,6 +6,7 @@
 #include "../../include/simp_gpu.h"
 
 #include "common.h"
+#include "conv_march.cuh"
 #include "conv_tc.cuh"
 #include "surrogate.h"
 #include "wgrad_tc.cuh"
@@ -58,15 +59,15 @@ void check_encode(CUresult r, const char* what) {
 
 }  // namespace
 
-// Channels-last BF16 activations [nz][ny][nx][c]: boxes of (c, 32, 4, 1).
-CUtensorMap act_map(const void* base, int c, int nx, int ny, int nz) {
+// Channels-last BF16 activations [nz][ny][nx][c]: boxes of (c, 32, rows, 1).
+CUtensorMap act_map(const void* base, int c, int nx, int ny, int nz, int rows) {
   if (reinterpret_cast<uintptr_t>(base) % 16) throw Error(kBadInput, "surrogate: activations must be 16-byte aligned");
   CUtensorMap m;
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(c), static_cast<cuuint64_t>(nx), static_cast<cuuint64_t>(ny),
                               static_cast<cuuint64_t>(nz)};
   const cuuint64_t strides[3] = {static_cast<cuuint64_t>(c) * 2, static_cast<cuuint64_t>(c) * 2 * nx,
                                  static_cast<cuuint64_t>(c) * 2 * nx * ny};
-  const cuuint32_t box[4] = {static_cast<cuuint32_t>(c), conv::kTileX, conv::kTileY, 1};
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(c), conv::kTileX, static_cast<cuuint32_t>(rows), 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   check_encode(encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_for(c * 2), CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -88,6 +89,39 @@ CUtensorMap weight_map(const void* base, int k, int n, int c) {
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE),
                "weights");
   return m;
+}
+
+// The marching kernel (conv_march.cuh) for the layers whose weights and two
+// loaded input layers fit in shared memory (the others, 64 and more input
+// channels, stay on k_conv_tc); false: not launched.
+static bool conv_march_launch(const ConvSpec& s, const conv::ConvArgs& p, int ktot, cudaStream_t stream) {
+  constexpr int kSmem = 216 * 1024;
+  int stages = conv::kMarchMaxStages;
+  while (stages > 1 && conv::march_smem(s.n, ktot, stages) > kSmem) --stages;
+  if (stages < 2 || s.n > 64) return false;
+  const int tx = (s.nx + conv::kTileX - 1) / conv::kTileX, ty = (s.ny + conv::kTileY - 1) / conv::kTileY;
+  conv::MarchArgs m{};
+  m.c = p;
+  m.w = static_cast<const __nv_bfloat16*>(s.w);
+  m.stages = stages;
+  // output layers a CTA holds in half of tensor memory (two CTAs an SM)
+  const int most = std::min(256 / s.n, conv::kMarchMaxSteps - 2);
+  const int chunks = (s.nz + most - 1) / most;
+  m.chunk = (s.nz + chunks - 1) / chunks;
+  const int smem = conv::march_smem(s.n, ktot, stages);
+  const CUtensorMap a0 = act_map(s.in[0], s.cseg[0], s.nx, s.ny, s.nz, conv::kMarchRows);
+  const CUtensorMap a1 = s.nseg > 1 ? act_map(s.in[1], s.cseg[1], s.nx, s.ny, s.nz, conv::kMarchRows) : a0;
+  auto launch = [&](auto kernel) {
+    raise_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<size_t>(smem));
+    kernel<<<dim3(tx, ty, (s.nz + m.chunk - 1) / m.chunk), conv::kMarchThreads, smem, stream>>>(a0, a1, m);
+    SIMP_CHECK_LAUNCH();
+    return true;
+  };
+  const int c1 = s.nseg > 1 ? s.cseg[1] : 0;
+  if (s.cseg[0] == 16 && c1 == 0) return s.flip ? launch(conv::k_conv_march<16, 0, true>) : launch(conv::k_conv_march<16, 0, false>);
+  if (s.cseg[0] == 32 && c1 == 0) return s.flip ? launch(conv::k_conv_march<32, 0, true>) : launch(conv::k_conv_march<32, 0, false>);
+  if (s.cseg[0] == 32 && c1 == 16 && !s.flip) return launch(conv::k_conv_march<32, 16, false>);
+  return false;
 }
 
 // One convolution (or its data gradient) on the tensor cores.
@@ -118,8 +152,9 @@ void conv_launch(const ConvSpec& s, cudaStream_t stream) {
     p.out[k] = s.out[k];
   }
   if (s.nout > 1 && s.out_c[0] % 16) throw Error(kBadInput, "surrogate: split outputs at a multiple of 16 columns");
-  const CUtensorMap a0 = act_map(s.in[0], s.cseg[0], s.nx, s.ny, s.nz);
-  const CUtensorMap a1 = s.nseg > 1 ? act_map(s.in[1], s.cseg[1], s.nx, s.ny, s.nz) : a0;
+  if (conv_march_launch(s, p, ktot, stream)) return;
+  const CUtensorMap a0 = act_map(s.in[0], s.cseg[0], s.nx, s.ny, s.nz, conv::kTileY);
+  const CUtensorMap a1 = s.nseg > 1 ? act_map(s.in[1], s.cseg[1], s.nx, s.ny, s.nz, conv::kTileY) : a0;
   const CUtensorMap b0 = weight_map(s.w, ktot, s.n, s.cseg[0]);
   const CUtensorMap b1 = s.nseg > 1 ? weight_map(s.w, ktot, s.n, s.cseg[1]) : b0;
   const size_t smem = conv::smem_bytes(p);
@@ -242,7 +277,10 @@ static void wgrad_tc_launch(const WgradSpec& s, float* part, cudaStream_t stream
   a.cdy = s.cdy;
   a.part = part;
   a.status = s.status;
-  a.run = static_cast<i64>(s.nx) * s.ny * s.nz <= (1 << 15) ? 2 : 4;
+  // longer accumulator runs on larger grids: fewer additions, and sums of more
+  // terms, to which a run's truncation adds less
+  const i64 nodes = static_cast<i64>(s.nx) * s.ny * s.nz;
+  a.run = nodes <= (1 << 13) ? 2 : nodes <= (1 << 15) ? 4 : 8;
   int nseg = 0, cmax = 0;
   auto add = [&](const __nv_bfloat16* x, int c, int ci0) {
     for (int k = 0; k < c; k += 32) {

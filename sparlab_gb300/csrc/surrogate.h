@@ -47,7 +47,7 @@ struct WgradSpec {
   int* status = nullptr;  // device word set on a wait that ran out
 };
 
-CUtensorMap act_map(const void* base, int c, int nx, int ny, int nz);
+CUtensorMap act_map(const void* base, int c, int nx, int ny, int nz, int rows);
 CUtensorMap weight_map(const void* base, int k, int n, int c);
 void conv_launch(const ConvSpec& s, cudaStream_t stream);
 void wgrad_launch(const WgradSpec& s, float* part, cudaStream_t stream);

@@ -21,11 +21,11 @@
 // The tensor core adds into its FP32 accumulator with truncation (about 0.4 x
 // 2^-24 of the sum per instruction, always towards zero), so a long sum
 // drifts: 3.6e-5 of the gradient over 193x97x97 nodes.  An accumulator
-// therefore takes four instructions (64 nodes) at a time and is then added to
-// FP32 registers, rounded to nearest, by the warps that own its rows; a ring
-// of four accumulator sets keeps the tensor core busy meanwhile.  Grids of up
-// to 2^15 nodes, whose gradients have fewer terms to average over and take a
-// launch's latency anyway, add after every second instruction.
+// therefore takes a run of up to eight instructions (a tile's 128 nodes) and is
+// then added to FP32 registers, rounded to nearest, by the warps that own its
+// rows; a ring of four accumulator sets keeps the tensor core busy meanwhile.
+// Small grids, whose gradients have fewer terms to average over, take shorter
+// runs (2 up to 2^13 nodes, 4 up to 2^15).
 //
 // Warps: 0, 4, 8 (and 1, 5, 9) add the accumulators (rows 32 (w % 4) .., a
 // third of the columns each), 6 issues the instructions, the others load.
@@ -33,11 +33,11 @@
 // of G walkers of the tiles; k_wgrad_tc_sum adds the G partials in order.
 //
 // Measured at 97x49x49 nodes, 16 -> 16 channels: 1,270 us on the CUDA cores
-// (FP32 multiply-adds from shared memory, two loads each), 80 us here (one
-// issuing warp of uniform control: 162 us when a single divergent thread
-// issued, about 70 cycles an instruction); bound by the issue of short runs,
-// 0.25 us each with their barriers.  Error of the gradient against FP64:
-// 3.8e-7 -> 1.7e-7 there, 7.9e-8 -> 4.6e-8 at 37x7x5.
+// (FP32 multiply-adds from shared memory, two loads each), 80 us with runs of
+// four here (one issuing warp of uniform control: 162 us when a single
+// divergent thread issued, about 70 cycles an instruction); bound by the
+// loads' latency and the runs' barriers (0.25 us a run).  Error of the
+// gradient against FP64: 3.8e-7 -> 1.5e-7 there, 7.9e-8 -> 4.6e-8 at 37x7x5.
 #pragma once
 
 #include "common.h"
@@ -72,7 +72,7 @@ struct Args {
   int cdy;  // 16, 32 or 64
   float* part;
   int* status;
-  int run;  // instructions an accumulator takes before it is added (2 or 4)
+  int run;  // instructions an accumulator takes before it is added (2, 4 or 8)
 };
 
 __host__ __device__ constexpr int stage_bytes(int cdy, int c) { return cdy / 8 * kPlaneY + 3 * (c / 8) * kPlaneX; }
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const Args p) {
   const int adders = p.cdy > 32 ? 6 : 3;
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
-      tc::mbar_init(&full[s], kLoaders);
+      tc::mbar_init(&full[s], kLoaders / 32);
       tc::mbar_init(&empty[s], 1);
     }
     for (int s = 0; s < kSets; ++s) {
@@ -217,11 +217,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const Args p) {
           const uint64_t a = a0 + part * p.run * 16, b = b0 + part * p.run * 16 + dy * kTX;
           if (leader) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)  // 16 nodes each
+            for (int k = 0; k < 8; ++k)  // 16 nodes each
               if (k < p.run) tc::mma_bf16(d, a + k * 16, b + k * 16, id, k != 0);
             if (bias && dy == 1)
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
+              for (int k = 0; k < 8; ++k)
                 if (k < p.run) tc::mma_bf16(d + 3 * sg.c, a + k * 16, bones, idb, k != 0);
             tc::mma_commit(&set_full[set]);
           }
@@ -283,7 +283,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_wgrad_tc(const Args p) {
       if (n >= 1) {  // tile n - 1 has landed: visible to the tensor core
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         tc::fence_proxy_async_smem();
-        mbar_arrive(&full[(n - 1) % kStages]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[(n - 1) % kStages]);
       }
     }
   }
