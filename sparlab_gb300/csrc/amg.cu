@@ -247,7 +247,6 @@ MfView mf_view(const MfOp& o) {
   v.nz = o.nz;
   v.nnx = o.nnx;
   v.nny = o.nny;
-  v.gnode = o.gnode;
   v.nindex = o.nindex;
   v.ke = o.ke;
   v.scale = o.scale;
@@ -383,66 +382,61 @@ void mf3(const MfOp& mf, const MfArgs& args, cudaStream_t s) {
   }
 }
 
-// Matrix-free level-0 pieces of the FP32 cycle (tiled in 3-D).
-void mf_cheb_first(const MfOp& mf, i32 nodes, const float* x, const float* b, float* r, float* d,
-                   const float* dinv, const float* inv_theta, cudaStream_t s) {
-  if (mf.dim == 3) {
-    MfArgs a{};
-    a.x = x;
-    a.b = b;
-    a.r = r;
-    a.dn = d;
-    a.dinv = dinv;
-    a.coef = inv_theta;
-    mf3<4>(mf, a, s);
-    return;
-  }
-  k_mf_cheb_first<<<grid_for(nodes, 256), 256, 0, s>>>(mf_view(mf), nodes, x, b, r, d, dinv, inv_theta);
+// Matrix-free level-0 pieces of the FP32 cycle.
+template <int MODE>
+void mf2(const MfOp& mf, const MfArgs& a, cudaStream_t s) {
+  KeQ4 ke;
+  std::copy(mf.ke_host, mf.ke_host + 8 * 8, ke.k);
+  const unsigned grid = static_cast<unsigned>((mf.nnx + 31) / 32) * static_cast<unsigned>((mf.nny + 3) / 4);
+  k_mf2<MODE><<<grid, 128, 0, s>>>(mf_view(mf), a.x, a.y, a.b, a.r, a.dn, a.xs, a.dinv, a.coef, a.add_d, ke);
   SIMP_CHECK_LAUNCH();
 }
 
-void mf_cheb_step(const MfOp& mf, i32 nodes, const float* d, const float* rin, float* r, float* dn, float* x,
-                  const float* dinv, const float* c12, int add_d, cudaStream_t s) {
-  if (mf.dim == 3) {
-    MfArgs a{};
-    a.x = d;
-    a.b = rin;
-    a.r = r;
-    a.dn = dn;
-    a.xs = x;
-    a.dinv = dinv;
-    a.coef = c12;
-    a.add_d = add_d;
-    mf3<3>(mf, a, s);
-    return;
-  }
-  k_mf_cheb_step<<<grid_for(nodes, 256), 256, 0, s>>>(mf_view(mf), nodes, d, rin, r, dn, x, dinv, c12, add_d);
-  SIMP_CHECK_LAUNCH();
+template <int MODE>
+void mf_product(const MfOp& mf, const MfArgs& a, cudaStream_t s) {
+  if (mf.dim == 3) mf3<MODE>(mf, a, s);
+  else mf2<MODE>(mf, a, s);
 }
 
-void mf_apply(const MfOp& mf, i32 nodes, const float* x, float* y, cudaStream_t s) {
-  if (mf.dim == 3) {
-    MfArgs a{};
-    a.x = x;
-    a.y = y;
-    mf3<0>(mf, a, s);
-    return;
-  }
-  k_mf_apply<0, float><<<grid_for(nodes, 256), 256, 0, s>>>(mf_view(mf), nodes, x, y, nullptr);
-  SIMP_CHECK_LAUNCH();
+void mf_cheb_first(const MfOp& mf, const float* x, const float* b, float* r, float* d, const float* dinv,
+                   const float* inv_theta, cudaStream_t s) {
+  MfArgs a{};
+  a.x = x;
+  a.b = b;
+  a.r = r;
+  a.dn = d;
+  a.dinv = dinv;
+  a.coef = inv_theta;
+  mf_product<4>(mf, a, s);
 }
 
-void mf_residual(const MfOp& mf, i32 nodes, const float* x, float* r, const float* b, cudaStream_t s) {
-  if (mf.dim == 3) {
-    MfArgs a{};
-    a.x = x;
-    a.y = r;
-    a.b = b;
-    mf3<1>(mf, a, s);
-    return;
-  }
-  k_mf_apply<1, float><<<grid_for(nodes, 256), 256, 0, s>>>(mf_view(mf), nodes, x, r, b);
-  SIMP_CHECK_LAUNCH();
+void mf_cheb_step(const MfOp& mf, const float* d, const float* rin, float* r, float* dn, float* x, const float* dinv,
+                  const float* c12, int add_d, cudaStream_t s) {
+  MfArgs a{};
+  a.x = d;
+  a.b = rin;
+  a.r = r;
+  a.dn = dn;
+  a.xs = x;
+  a.dinv = dinv;
+  a.coef = c12;
+  a.add_d = add_d;
+  mf_product<3>(mf, a, s);
+}
+
+void mf_apply(const MfOp& mf, const float* x, float* y, cudaStream_t s) {
+  MfArgs a{};
+  a.x = x;
+  a.y = y;
+  mf_product<0>(mf, a, s);
+}
+
+void mf_residual(const MfOp& mf, const float* x, float* r, const float* b, cudaStream_t s) {
+  MfArgs a{};
+  a.x = x;
+  a.y = r;
+  a.b = b;
+  mf_product<1>(mf, a, s);
 }
 
 // Level-0 transfers of the FP32 cycle without the stored R and P
@@ -766,13 +760,13 @@ void GpuAmg::spmv0_fast(const double* x, double* y) {
   LevelWork& v = work(0).lv.front();  // the cycle's level-0 vectors are free between solves
   if (mf.planes) {
     to_planes(x, v.d32.p, l0.nnodes, stream);
-    mf_apply(mf, l0.nnodes, v.d32.p, v.e32.p, stream);
+    mf_apply(mf, v.d32.p, v.e32.p, stream);
     from_planes(v.e32.p, y, l0.nnodes, stream);
     return;
   }
   convert(x, v.d32.p, n, stream);
   if (mf.enabled) {
-    mf_apply(mf, l0.nnodes, v.d32.p, v.e32.p, stream);
+    mf_apply(mf, v.d32.p, v.e32.p, stream);
   } else {
     nb_apply<0, float, float, float>(l0.opA, l0.a.v32.p, v.d32.p, v.e32.p, nullptr, stream);
   }
@@ -888,7 +882,7 @@ void GpuAmg::lanczos(size_t l, int m, double* ab) {
   SIMP_CHECK_LAUNCH();
   for (int j = 0; j < m; ++j) {
     if constexpr (std::is_same<T, float>::value) {
-      if (l == 0 && mf.enabled) mf_apply(mf, lv.nnodes, tmp, w, stream);
+      if (l == 0 && mf.enabled) mf_apply(mf, tmp, w, stream);
       else nb_apply<0, float, float, float>(lv.opA, lv.a.v32.p, tmp, w, nullptr, stream);
     } else {
       nb_apply<0, double, double, double>(lv.opA, lv.a.v64.p, tmp, w, nullptr, stream);
@@ -1537,7 +1531,7 @@ void GpuAmg::smooth(SolveWork& w, size_t l, bool zero_guess) {
     SIMP_CHECK_LAUNCH();
   } else if (matrix_free) {
     if constexpr (std::is_same<T, float>::value)
-      mf_cheb_first(mf, lv.nnodes, x, b, r, d, dinv, lv.cheb32.p, stream);
+      mf_cheb_first(mf, x, b, r, d, dinv, lv.cheb32.p, stream);
   } else {
     nb_cheb_first<T>(lv.opA, A, x, b, r, d, dinv, V<T>::cheb(lv), stream);
   }
@@ -1546,7 +1540,7 @@ void GpuAmg::smooth(SolveWork& w, size_t l, bool zero_guess) {
     const int add_d = (k == 1 && !zero_guess) ? 1 : 0;
     if (matrix_free) {
       if constexpr (std::is_same<T, float>::value)
-        mf_cheb_step(mf, lv.nnodes, d, rin, r, e, x, dinv, lv.cheb32.p + 2 * k - 1, add_d, stream);
+        mf_cheb_step(mf, d, rin, r, e, x, dinv, lv.cheb32.p + 2 * k - 1, add_d, stream);
     } else {
       nb_cheb_step<T>(lv.opA, A, d, rin, r, e, x, dinv, V<T>::cheb(lv) + 2 * k - 1, add_d, stream);
     }
@@ -1581,7 +1575,7 @@ void GpuAmg::cycle(SolveWork& w, size_t l) {
   }
   if (matrix_free) {  // residual
     if constexpr (std::is_same<T, float>::value)
-      mf_residual(mf, lv.nnodes, V<T>::x(v), V<T>::r(v), V<T>::b(v), stream);
+      mf_residual(mf, V<T>::x(v), V<T>::r(v), V<T>::b(v), stream);
   } else {
     nb_apply<1, T, T, T>(lv.opA, V<T>::a(lv.a), V<T>::x(v), V<T>::r(v), V<T>::b(v), stream);
   }

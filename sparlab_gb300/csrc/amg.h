@@ -146,7 +146,6 @@ struct MfOp {
   bool enabled = false;
   int dim = 3;
   i32 nx = 0, ny = 0, nz = 1, nnx = 0, nny = 0;
-  const i32* gnode = nullptr;   // free node -> grid node
   const i32* nindex = nullptr;  // grid node -> free node or -1
   const float* ke = nullptr;    // K_e^0, FP32
   const float* scale = nullptr; // s_e, FP32

@@ -19,122 +19,111 @@ struct MfView {
   int dim;             // 2 or 3
   i32 nx, ny, nz;      // cells (nz = 1 in 2-D)
   i32 nnx, nny;        // nodes per axis in x, y
-  const i32* gnode;    // free node -> grid node
   const i32* nindex;   // grid node -> free node or -1
   const float* ke;     // K_e^0 (ed x ed, row-major)
   const float* scale;  // s_e
 };
 
-// Per-node product (A x)_I for the free node I; out[k], k < dim.
-template <class TX>
-__device__ __forceinline__ void mf_node_apply(const MfView& m, const float* __restrict__ ks, i32 I,
-                                              const TX* __restrict__ x, float (&out)[3]) {
-  const int dim = m.dim;
-  const int ed = dim == 3 ? 24 : 8;
-  out[0] = out[1] = out[2] = 0.0f;
-  const i32 g = m.gnode[I];
-  const i32 ix = g % m.nnx, iy = (g / m.nnx) % m.nny, iz = g / (m.nnx * m.nny);
-  const int zlo = dim == 3 ? -1 : 0;
-  for (int dz = zlo; dz <= 0; ++dz)
-    for (int dy = -1; dy <= 0; ++dy)
-      for (int dx = -1; dx <= 0; ++dx) {
-        const i32 cx = ix + dx, cy = iy + dy, cz = iz + dz;
-        if (cx < 0 || cx >= m.nx || cy < 0 || cy >= m.ny || cz < 0 || cz >= m.nz) continue;
-        const float s = m.scale[(static_cast<i64>(cz) * m.ny + cy) * m.nx + cx];
-        // corner index of node I in cell c: offsets (-dx, -dy, -dz)
-        const int ox = -dx, oy = -dy, oz = -dz;
-        const int aI = 4 * oz + (oy ? 3 - ox : ox);
-        float acc[3] = {0.0f, 0.0f, 0.0f};
-        const int npe = dim == 3 ? 8 : 4;
-        for (int b = 0; b < npe; ++b) {
-          const int bx = (b == 1 || b == 2 || b == 5 || b == 6) ? 1 : 0;
-          const int by = (b == 2 || b == 3 || b == 6 || b == 7) ? 1 : 0;
-          const int bz = b >= 4 ? 1 : 0;
-          const i64 gj = (static_cast<i64>(cz + bz) * m.nny + (cy + by)) * m.nnx + (cx + bx);
-          const i32 J = m.nindex[gj];
-          if (J < 0) continue;
-          float xj[3];
+// ---------------------------------------------------------------------------
+// 2-D operator: one thread per grid node (32 x 4 nodes a block), K_e^0 a
+// kernel parameter indexed by compile-time constants.  Every index, then every
+// value and scale of the 3 x 3 neighbourhood is loaded before the first
+// product: two load latencies a thread, which bound the kernel at the sizes of
+// 2-D problems (against a loop over cells and corners with a division-decoded
+// node index, 11.6 us a Chebyshev step at 120x40 cells, a SIMP iteration went
+// from 4.85 to 4.27 ms there and from 10.6 to 9.4 ms at 600x200 with three load
+// cases; the products and their order are the same).  Modes as in k_mf3_tile:
+// 0 y = A x, 1 y = b - A x, 3 Chebyshev step, 4 Chebyshev first step.
+// ---------------------------------------------------------------------------
+struct KeQ4 {
+  float k[8 * 8];  // K_e^0, row-major
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(128) k_mf2(MfView m, const float* __restrict__ x, float* __restrict__ y,
+                                             const float* b, float* r, float* __restrict__ dn, float* xs,
+                                             const float* __restrict__ dinv, const float* __restrict__ coef, int add_d,
+                                             const __grid_constant__ KeQ4 ke) {
+  const i32 across = (m.nnx + 31) / 32;  // blocks of a row of blocks
+  const i32 ix = blockIdx.x % across * 32 + (threadIdx.x & 31), iy = blockIdx.x / across * 4 + (threadIdx.x >> 5);
+  if (ix >= m.nnx || iy >= m.nny) return;
+  i32 J[3][3];
+  float s[2][2];
 #pragma unroll
-          for (int k = 0; k < 3; ++k) xj[k] = k < dim ? static_cast<float>(x[static_cast<i64>(J) * dim + k]) : 0.0f;
+  for (int v = 0; v < 3; ++v)
 #pragma unroll
-          for (int ka = 0; ka < 3; ++ka) {
-            if (ka < dim) {
-              const float* row = ks + (dim * aI + ka) * ed + dim * b;
+    for (int u = 0; u < 3; ++u) {
+      const i32 jx = ix + u - 1, jy = iy + v - 1;
+      J[v][u] = jx >= 0 && jx < m.nnx && jy >= 0 && jy < m.nny ? m.nindex[static_cast<i64>(jy) * m.nnx + jx] : -1;
+    }
 #pragma unroll
-              for (int kb = 0; kb < 3; ++kb)
-                if (kb < dim) acc[ka] = fmaf(row[kb], xj[kb], acc[ka]);
-            }
-          }
-        }
+  for (int v = 0; v < 2; ++v)
 #pragma unroll
-        for (int ka = 0; ka < 3; ++ka) out[ka] = fmaf(s, acc[ka], out[ka]);
+    for (int u = 0; u < 2; ++u) {
+      const i32 cx = ix + u - 1, cy = iy + v - 1;
+      s[v][u] = cx >= 0 && cx < m.nx && cy >= 0 && cy < m.ny ? m.scale[static_cast<i64>(cy) * m.nx + cx] : 0.0f;
+    }
+  const i32 I = J[1][1];
+  if (I < 0) return;
+  float2 xv[3][3];
+#pragma unroll
+  for (int v = 0; v < 3; ++v)
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      xv[v][u] = J[v][u] >= 0 ? reinterpret_cast<const float2*>(x)[J[v][u]] : make_float2(0.0f, 0.0f);
+  // the epilogue's operands are in flight during the products
+  const i64 row = 2 * static_cast<i64>(I);
+  float bi[2] = {}, di[2] = {}, xi[2] = {}, c0 = 0.0f, c1 = 0.0f;
+  if (MODE != 0) {
+    bi[0] = b[row];
+    bi[1] = b[row + 1];
+  }
+  if (MODE == 3 || MODE == 4) {
+    di[0] = dinv[row];
+    di[1] = dinv[row + 1];
+    c0 = coef[0];
+  }
+  if (MODE == 3) {
+    c1 = coef[1];
+    xi[0] = xs[row];
+    xi[1] = xs[row + 1];
+  }
+  float out[2] = {0.0f, 0.0f};
+#pragma unroll
+  for (int v = 0; v < 2; ++v)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {  // cell (ix + u - 1, iy + v - 1); this node is its corner (1 - u, 1 - v)
+      const int ox = 1 - u, oy = 1 - v, a = oy ? 3 - ox : ox;
+      float acc[2] = {0.0f, 0.0f};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int bx = c == 1 || c == 2, by = c >= 2;
+        const float2 t = xv[v + by][u + bx];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          acc[k] = fmaf(ke.k[(2 * a + k) * 8 + 2 * c + 1], t.y, fmaf(ke.k[(2 * a + k) * 8 + 2 * c], t.x, acc[k]));
       }
-}
-
-// mode 0: y = A x ; 1: y = b - A x ; 2: y += A x
-template <int MODE, class TX>
-__global__ void __launch_bounds__(256) k_mf_apply(MfView m, i32 nodes, const TX* __restrict__ x, TX* __restrict__ y,
-                                                  const TX* __restrict__ b) {
-  __shared__ float ks[24 * 24];
-  const int ed = m.dim == 3 ? 24 : 8;
-  for (int k = threadIdx.x; k < ed * ed; k += blockDim.x) ks[k] = m.ke[k];
-  __syncthreads();
-  const i32 I = blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= nodes) return;
-  float out[3];
-  mf_node_apply<TX>(m, ks, I, x, out);
-  for (int k = 0; k < m.dim; ++k) {
-    const i64 row = static_cast<i64>(I) * m.dim + k;
-    if (MODE == 0) y[row] = static_cast<TX>(out[k]);
-    else if (MODE == 1) y[row] = b[row] - static_cast<TX>(out[k]);
-    else y[row] += static_cast<TX>(out[k]);
-  }
-}
-
-// Chebyshev step: r = r_in - A d ; dn = c1 d + c2 dinv r ; x = (x [+ d]) + dn
-__global__ void __launch_bounds__(256) k_mf_cheb_step(MfView m, i32 nodes, const float* __restrict__ d,
-                                                      const float* __restrict__ r_in, float* __restrict__ r,
-                                                      float* __restrict__ dn, float* __restrict__ x,
-                                                      const float* __restrict__ dinv,
-                                                      const float* __restrict__ c12, int add_d) {
-  __shared__ float ks[24 * 24];
-  const int ed = m.dim == 3 ? 24 : 8;
-  for (int k = threadIdx.x; k < ed * ed; k += blockDim.x) ks[k] = m.ke[k];
-  __syncthreads();
-  const i32 I = blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= nodes) return;
-  float out[3];
-  mf_node_apply<float>(m, ks, I, d, out);
-  for (int k = 0; k < m.dim; ++k) {
-    const i64 row = static_cast<i64>(I) * m.dim + k;
-    const float ri = r_in[row] - out[k];
-    r[row] = ri;
-    const float di = c12[0] * d[row] + c12[1] * dinv[row] * ri;
-    dn[row] = di;
-    float xi = x[row];
-    if (add_d) xi = xi + d[row];
-    x[row] = xi + di;
-  }
-}
-
-// r = b - A x ; d = dinv r / theta
-__global__ void __launch_bounds__(256) k_mf_cheb_first(MfView m, i32 nodes, const float* __restrict__ x,
-                                                       const float* __restrict__ b, float* __restrict__ r,
-                                                       float* __restrict__ d, const float* __restrict__ dinv,
-                                                       const float* __restrict__ inv_theta) {
-  __shared__ float ks[24 * 24];
-  const int ed = m.dim == 3 ? 24 : 8;
-  for (int k = threadIdx.x; k < ed * ed; k += blockDim.x) ks[k] = m.ke[k];
-  __syncthreads();
-  const i32 I = blockIdx.x * blockDim.x + threadIdx.x;
-  if (I >= nodes) return;
-  float out[3];
-  mf_node_apply<float>(m, ks, I, x, out);
-  for (int k = 0; k < m.dim; ++k) {
-    const i64 row = static_cast<i64>(I) * m.dim + k;
-    const float ri = b[row] - out[k];
-    r[row] = ri;
-    d[row] = dinv[row] * ri * *inv_theta;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) out[k] = fmaf(s[v][u], acc[k], out[k]);
+    }
+  const float self[2] = {xv[1][1].x, xv[1][1].y};
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (MODE == 0) {
+      y[row + k] = out[k];
+    } else if (MODE == 1) {
+      y[row + k] = bi[k] - out[k];
+    } else {
+      const float ri = bi[k] - out[k];
+      r[row + k] = ri;
+      if (MODE == 4) {
+        dn[row + k] = di[k] * ri * c0;
+      } else {
+        const float dv = c0 * self[k] + c1 * di[k] * ri;
+        dn[row + k] = dv;
+        xs[row + k] = (add_d ? xi[k] + self[k] : xi[k]) + dv;
+      }
+    }
   }
 }
 

@@ -267,7 +267,6 @@ void GpuProblem::build() {
       mf.nz = d.nz;
       mf.nnx = g.nnx;
       mf.nny = g.nny;
-      mf.gnode = gnode.p;
       mf.nindex = nindex.p;
       mf.ke = ke32.p;
       std::copy(k32.begin(), k32.end(), mf.ke_host);
