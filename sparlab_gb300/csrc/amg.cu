@@ -60,37 +60,6 @@ __global__ void k_expand_columns(i32 n, const i32* __restrict__ node_of, NodeVie
 
 namespace {
 
-// w = s .* w - beta vp (beta from device memory); nothing once stopped.
-// FP64 vectors: FP64 arithmetic; FP32 vectors (the reuse setups): FP32
-// arithmetic, with beta rounded to FP32 (GB300 runs FP64 at 1/64 of the
-// FP32 rate, so conversions and FP64 operations per element would bound
-// these vector passes)
-template <class T>
-__global__ void k_lanczos_finish(T* __restrict__ w, const T* __restrict__ s, const T* __restrict__ vp,
-                                 const double* __restrict__ beta, const double* __restrict__ stop, i64 n) {
-  if (*stop != 0.0) return;
-  const double bj = vp ? *beta : 0.0;
-  if constexpr (std::is_same<T, float>::value) {
-    const float bf = static_cast<float>(bj);
-    for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-      float wi = w[i] * s[i];
-      if (vp) wi = fmaf(-bf, vp[i], wi);
-      w[i] = wi;
-    }
-  } else {
-    for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-      double wi = todbl(w[i]) * todbl(s[i]);
-      if (vp) wi -= bj * todbl(vp[i]);
-      w[i] = static_cast<T>(wi);
-    }
-  }
-}
-
-// The reference's breakdown test of step j: stop when beta_j <= 1e-12 |alpha_j|
-__global__ void k_lanczos_check(const double* __restrict__ ab, int j, double* __restrict__ stop) {
-  if (threadIdx.x == 0 && blockIdx.x == 0 && !(ab[2 * j + 1] > 1.0e-12 * fabs(ab[2 * j]))) *stop = 1.0;
-}
-
 // Every operator application runs the VS-lanes-per-row kernels of
 // nbspmv.cuh; (VS, B) come from the operator's shape: B = the uniform width of
 // its column nodes (column-free decode) or 0, VS = the lanes per row chosen
@@ -130,6 +99,10 @@ void with_shape_df(const NbOp& op, F&& f) {
     default: lanes(std::integral_constant<int, 0>{}); break;
   }
 }
+
+// Blocks of a grid-stride reduction over n values: at most kRedBlocks, fewer
+// where a block would have less than one value a thread.
+int red_blocks(i64 n) { return grid_for(n, kRedThreads, kRedBlocks); }
 
 // One thread per (row, lane); no grid-stride loop in the row kernels.
 unsigned rows_grid(const NbOp& op, int vs) {
@@ -860,48 +833,57 @@ struct LzBufs<float> {
   static DBuf<float>* get(Level& l) { return l.lz32; }
 };
 
-// The m Lanczos steps of a level (Multigrid.cpp:288-327).  T = double: FP64
-// vectors and operator.  T = float (the FP32 reuse setups): FP32 vectors and
-// the FP32 operator the smoother uses (matrix-free on a structured level 0),
-// with the scalars and the sums of the dot products in FP64.
+// Inverse diagonal and the m Lanczos steps of a level (Multigrid.cpp:288-327,
+// 718-747).  T = double: FP64 vectors and operator.  T = float (the FP32 reuse
+// setups): FP32 vectors and the FP32 operator the smoother uses (matrix-free
+// on a structured level 0), with the scalars and the sums across warps in
+// FP64.
 template <class T>
 void GpuAmg::lanczos(size_t l, int m, double* ab) {
   Level& lv = *levels[l];
   const i32 n = lv.n;
-  double* stop = ab + 2 * m;
+  constexpr bool f32 = std::is_same<T, float>::value;
   DBuf<T>* bufs = LzBufs<T>::get(lv);
-  for (int k = 0; k < 5; ++k) bufs[k].alloc(static_cast<size_t>(n));
+  for (int k = 0; k < 4; ++k) bufs[k].alloc(static_cast<size_t>(n));
   T* v = bufs[0].p;
-  T* vp = bufs[1].p;
-  T* w = bufs[2].p;
-  T* s = bufs[3].p;
-  T* tmp = bufs[4].p;
-  const i64 planes = l == 0 && mf.planes ? lv.nnodes : 0;
-  k_lanczos_start<T><<<grid_for(n, 256), 256, 0, stream>>>(lv.lz_start.p, v, scal.p + 1, lv.dinv64.p, s, tmp, n,
-                                                          planes);
+  T* w = bufs[1].p;
+  T* s = bufs[2].p;
+  T* t = bufs[3].p;
+  const T* values = V<T>::a(lv.a);
+  LzScalars* sc = reinterpret_cast<LzScalars*>(ab + 2 * m);
+  const bool matrix_free = f32 && l == 0 && mf.enabled;
+  const i64 planes = matrix_free && mf.planes ? lv.nnodes : 0;
+  const int vs = f32 ? lv.opA.lanes32 : lv.opA.lanes64;
+  lz_part_.alloc(std::max<size_t>(lz_part_.n, std::max<size_t>(kRedBlocks, rows_grid(lv.opA, vs))));
+  double* pt = lz_part_.p;
+  k_lz_reset<<<1, 1, 0, stream>>>(sc, lv.lz_norm);
   SIMP_CHECK_LAUNCH();
+  // (level 0's dinv32 after a first setup follows when its order is known)
+  if (mixed()) lv.dinv32.alloc(n);
+  k_level_start<T><<<grid_for(n, 256), 256, 0, stream>>>(n, lv.d_node_of.p, lv.d_first.p, lv.d_self.p,
+                                                         lv.d_apat.view(), lv.a.ptr.p, values, lv.lz_start.p,
+                                                         lv.dinv64.p, lv.dinv32.p, s, w, t, v, planes, sc);
+  SIMP_CHECK_LAUNCH();
+  if constexpr (f32)
+    if (matrix_free) lz_y_.alloc(static_cast<size_t>(n));
+  const int blocks = red_blocks(n);
   for (int j = 0; j < m; ++j) {
-    if constexpr (std::is_same<T, float>::value) {
-      if (l == 0 && mf.enabled) mf_apply(mf, tmp, w, stream);
-      else nb_apply<0, float, float, float>(lv.opA, lv.a.v32.p, tmp, w, nullptr, stream);
+    if (matrix_free) {
+      if constexpr (f32) {
+        mf_apply(mf, t, lz_y_.p, stream);
+        k_lz_post<float><<<blocks, kRedThreads, 0, stream>>>(lz_y_.p, s, w, v, n, ab + 2 * j, pt, sc);
+        SIMP_CHECK_LAUNCH();
+      }
     } else {
-      nb_apply<0, double, double, double>(lv.opA, lv.a.v64.p, tmp, w, nullptr, stream);
+      with_shape<T>(lv.opA, [&](auto lanes, auto blk) {
+        constexpr int VS = decltype(lanes)::value, B = decltype(blk)::value;
+        k_lz_rows<VS, B, T><<<rows_grid(lv.opA, VS), 256, 0, stream>>>(n, lv.opA.node_of, lv.opA.pat, lv.opA.rowptr,
+                                                                       lv.opA.col, values, t, s, w, v, ab + 2 * j, pt, sc);
+      });
+      SIMP_CHECK_LAUNCH();
     }
-    k_lanczos_finish<T><<<grid_for(n, 256), 256, 0, stream>>>(w, s, j > 0 ? vp : nullptr,
-                                                             j > 0 ? ab + 2 * j - 1 : nullptr, stop, n);
-    SIMP_CHECK_LAUNCH();
-    k_dot_partial<T, T><<<kRedBlocks, kRedThreads, 0, stream>>>(w, v, n, part.p);
-    SIMP_CHECK_LAUNCH();
-    k_reduce_final<<<1, kRedThreads, 0, stream>>>(part.p, kRedBlocks, ab + 2 * j, 0);
-    SIMP_CHECK_LAUNCH();
     if (j + 1 == m) break;  // beta of the last step is not used
-    k_axpy_norm<T><<<kRedBlocks, kRedThreads, 0, stream>>>(w, v, ab + 2 * j, n, part.p);
-    SIMP_CHECK_LAUNCH();
-    k_reduce_final<<<1, kRedThreads, 0, stream>>>(part.p, kRedBlocks, ab + 2 * j + 1, 1);
-    SIMP_CHECK_LAUNCH();
-    k_lanczos_check<<<1, 32, 0, stream>>>(ab, j, stop);
-    SIMP_CHECK_LAUNCH();
-    k_lanczos_shift<T><<<grid_for(n, 256), 256, 0, stream>>>(v, vp, w, s, tmp, ab + 2 * j + 1, stop, n);
+    k_lz_norm<T><<<blocks, kRedThreads, 0, stream>>>(s, w, v, t, n, ab + 2 * j, pt, sc);
     SIMP_CHECK_LAUNCH();
   }
 }
@@ -913,26 +895,10 @@ void GpuAmg::numeric_level(size_t l) {
   const bool fp32 = mixed() && ready_ && lv.a.v32.p != nullptr;
   make_ops(l);
   lv.dinv64.alloc(n);
-  SIMP_CUDA(cudaMemsetAsync(dstatus.p, 0x7f, sizeof(int), stream));
-  if (fp32)
-    k_inv_diag<float><<<grid_for(n, 256), 256, 0, stream>>>(n, lv.d_node_of.p, lv.d_first.p, lv.d_self.p,
-                                                            lv.d_apat.view(), lv.a.ptr.p, lv.a.v32.p, lv.dinv64.p,
-                                                            dstatus.p);
-  else
-    k_inv_diag<double><<<grid_for(n, 256), 256, 0, stream>>>(n, lv.d_node_of.p, lv.d_first.p, lv.d_self.p,
-                                                             lv.d_apat.view(), lv.a.ptr.p, lv.a.v64.p, lv.dinv64.p,
-                                                             dstatus.p);
-  SIMP_CHECK_LAUNCH();
-  // the diagonal's status is read with the Lanczos coefficients below (one
-  // host round trip per level); a bad diagonal only makes them garbage
-  if (mixed() && l > 0) {  // (level 0's copy follows when its vectors' order is known)
-    lv.dinv32.alloc(n);
-    convert(lv.dinv64.p, lv.dinv32.p, n, stream);
-  }
   // Lanczos on D^-1/2 A D^-1/2 with the reference's start vector (its norm
-  // made once per size); alpha_j, beta_j stay in device memory (lz_ab_[2j],
-  // [2j+1]; [2m] = the stop flag of the breakdown test): the steps after a
-  // breakdown change nothing, and the host reads all coefficients once
+  // made once per size); the scalars stay in device memory: the steps after a
+  // breakdown change nothing, and the host reads all coefficients and the
+  // diagonal's status once (a bad diagonal only makes them garbage)
   if (lv.lz_start.n != static_cast<size_t>(n)) {
     std::vector<double> h(static_cast<size_t>(n));
     for (i32 i = 0; i < n; ++i) h[i] = 1.0 + 0.5 * std::sin(1.7 * static_cast<double>(i) + 0.3);
@@ -940,20 +906,19 @@ void GpuAmg::numeric_level(size_t l) {
     lv.lz_norm = std::sqrt(dot(lv.lz_start.p, lv.lz_start.p, n));
   }
   const int m = std::max(1, std::min<int>(opt.lanczos_steps, n));
-  lz_ab_.alloc(static_cast<size_t>(2 * m + 1));
-  double* ab = lz_ab_.p;
-  SIMP_CUDA(cudaMemsetAsync(ab + 2 * m, 0, sizeof(double), stream));
-  SIMP_CUDA(cudaMemcpyAsync(scal.p + 1, &lv.lz_norm, sizeof(double), cudaMemcpyHostToDevice, stream));
-  if (fp32) lanczos<float>(l, m, ab);
-  else lanczos<double>(l, m, ab);
-  int bad = 0;
-  std::vector<double> hab(static_cast<size_t>(2 * m));
-  SIMP_CUDA(cudaMemcpyAsync(hab.data(), ab, sizeof(double) * 2 * m, cudaMemcpyDeviceToHost, stream));
-  SIMP_CUDA(cudaMemcpyAsync(&bad, dstatus.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  // alpha_j, beta_j pairs, then the scalars
+  const size_t words = 2 * static_cast<size_t>(m) + sizeof(LzScalars) / sizeof(double);
+  lz_ab_.alloc(std::max(lz_ab_.n, words));
+  lz_host_.alloc(words);
+  if (fp32) lanczos<float>(l, m, lz_ab_.p);
+  else lanczos<double>(l, m, lz_ab_.p);
+  const double* hab = lz_host_.p;
+  SIMP_CUDA(cudaMemcpyAsync(lz_host_.p, lz_ab_.p, sizeof(double) * words, cudaMemcpyDeviceToHost, stream));
   SIMP_CUDA(cudaStreamSynchronize(stream));
-  if (bad != 0x7f7f7f7f) {
+  const LzScalars& h = *reinterpret_cast<const LzScalars*>(hab + 2 * m);
+  if (h.bad != kLzGood) {
     std::ostringstream os;
-    os << "multigrid level " << l << ": diagonal entry " << bad
+    os << "multigrid level " << l << ": diagonal entry " << h.bad
        << " is not positive; a stiffness matrix must have a positive diagonal. The model has an "
           "unconnected degree of freedom or a non-positive stiffness";
     throw Error(kBreakdown, os.str());
@@ -996,11 +961,24 @@ void GpuAmg::numeric_level(size_t l) {
   }
   coef.push_back(0.0);
   coef.push_back(0.0);
-  const std::vector<float> coef32(coef.begin(), coef.end());
-  lv.cheb64.upload(coef, stream);
-  lv.cheb32.upload(coef32, stream);
-  const std::vector<float> omega{static_cast<float>(opt.damping / lv.lambda)};
-  lv.omega32.upload(omega, stream);
+  const double omega = opt.damping / lv.lambda;
+  lv.cheb64.alloc(coef.size());
+  lv.cheb32.alloc(coef.size());
+  lv.omega32.alloc(1);
+  ChebValues cv{};
+  if (coef.size() <= sizeof(cv.v) / sizeof(cv.v[0])) {  // as kernel arguments: no copy from pageable memory
+    std::copy(coef.begin(), coef.end(), cv.v);
+    cv.count = static_cast<int>(coef.size());
+    cv.omega = omega;
+    k_set_cheb<<<1, 64, 0, stream>>>(cv, lv.cheb64.p, lv.cheb32.p, lv.omega32.p);
+    SIMP_CHECK_LAUNCH();
+  } else {
+    const std::vector<float> coef32(coef.begin(), coef.end());
+    lv.cheb64.upload(coef, stream);
+    lv.cheb32.upload(coef32, stream);
+    const std::vector<float> omega32{static_cast<float>(omega)};
+    lv.omega32.upload(omega32, stream);
+  }
 }
 
 // Aggregates, tentative prolongator and symbolic patterns of level l -> l+1.
@@ -1398,9 +1376,7 @@ void GpuAmg::setup(bool structure_changed) {
     mf.free_nodes = l0.nnodes;
     mf.planes = mf.enabled && mf.dim == 3 && mf.parity && !mf.tensor && opt.mf_transfer && levels.size() > 1 &&
                 l0.mf_transfer && mf.grid_nodes() >= kParCycleNodes;
-    l0.dinv32.alloc(static_cast<size_t>(l0.n));
-    if (mf.planes) to_planes(l0.dinv64.p, l0.dinv32.p, l0.nnodes, stream);
-    else convert(l0.dinv64.p, l0.dinv32.p, l0.n, stream);
+    if (mf.planes && !fp32) to_planes(l0.dinv64.p, l0.dinv32.p, l0.nnodes, stream);
   }
   coarse_factorize();
   ensure(main_);

@@ -124,8 +124,8 @@ struct Level {
   DBuf<float> raw32;
   std::vector<double> c1, c2;
   double inv_theta = 0.0;
-  DBuf<double> lz[5];  // Lanczos work vectors (FP64 setups)
-  DBuf<float> lz32[5];  // (FP32 reuse setups)
+  DBuf<double> lz[4];  // Lanczos work vectors (FP64 setups)
+  DBuf<float> lz32[4];  // (FP32 reuse setups)
   DBuf<double> lz_start;  // Lanczos start vector (depends on n only) and its norm
   double lz_norm = 0.0;
 };
@@ -319,7 +319,10 @@ class GpuAmg {
  private:
   bool ready_ = false;
   i32 nc_ = 0;
-  DBuf<double> lz_ab_;  // Lanczos coefficients of the level in setup, and its stop flag
+  DBuf<double> lz_ab_;        // Lanczos coefficients and scalars of the level in setup
+  PinnedBuf<double> lz_host_;
+  DBuf<double> lz_part_;      // block partials of its sums
+  DBuf<float> lz_y_;          // the matrix-free product of a step
   DBuf<double> dense_, swept_, piv_, panel_;  // A_c^-1 (full), the sweep's lower triangle, pivots, U/V/P
   SolveWork main_;
   std::vector<std::unique_ptr<SolveWork>> extra_;

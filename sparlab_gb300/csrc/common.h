@@ -96,6 +96,28 @@ struct DBuf {
   size_t bytes() const { return n * sizeof(T); }
 };
 
+// Owning page-locked host array (copies to and from it do not pass through the
+// driver's staging).
+template <class T>
+struct PinnedBuf {
+  T* p = nullptr;
+  size_t n = 0;
+  PinnedBuf() = default;
+  PinnedBuf(const PinnedBuf&) = delete;
+  PinnedBuf& operator=(const PinnedBuf&) = delete;
+  ~PinnedBuf() {
+    if (p) cudaFreeHost(p);
+  }
+  void alloc(size_t count) {
+    if (p && count <= n) return;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    n = 0;
+    SIMP_CUDA(cudaMallocHost(&p, count * sizeof(T)));
+    n = count;
+  }
+};
+
 // Raises a kernel's dynamic shared-memory limit to at least `bytes` and never
 // lowers it: the limit is one value per kernel, shared by every host thread,
 // so a thread that set a smaller value could make another thread's larger

@@ -127,6 +127,31 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;
 }
 
+// Sum over the grid of one double per block (valid in thread 0): every block
+// stores its partial and takes a ticket, and the last one adds the partials in
+// order, so the value does not depend on which block that is.  True in that
+// block's thread 0, with the total; the ticket is back at zero for the next
+// launch.
+__device__ __forceinline__ bool grid_sum(double block, double* __restrict__ part, unsigned* __restrict__ ticket,
+                                         double& total) {
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = block;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  double s = 0.0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += 256) s += __ldcg(part + i);
+  s = block_sum<256>(s);
+  if (threadIdx.x != 0) return false;
+  *ticket = 0u;
+  total = s;
+  return true;
+}
+
 // ---------------------------------------------------------------------------
 // elementwise
 // ---------------------------------------------------------------------------
@@ -285,107 +310,152 @@ __global__ void k_cheb_zero(i64 n, const TX* __restrict__ b, const TX* __restric
 }
 
 // ---------------------------------------------------------------------------
-// Lanczos pieces (src/fem/Multigrid.cpp:288-327)
+// Lanczos on S A S, S = D^-1/2 (src/fem/Multigrid.cpp:288-327), two launches a
+// step instead of eight: the operator's rows with the step's vector update and
+// the partial sums of alpha_j in their epilogue (k_lz_rows, or a matrix-free
+// product and k_lz_post), then k_lz_norm; the last block of each adds the
+// partials in order.  The vector of a step stays unnormalised: u = beta_{j-1}
+// v_j is in w and t = s u is the operator's input, scaled in the rows'
+// epilogue, so no pass divides by beta.  FP32 vectors (the mixed-precision
+// reuse setups) take FP32 arithmetic with FP64 scalars and sums across warps:
+// GB300 runs FP64 at 1/64 of the FP32 rate.
 // ---------------------------------------------------------------------------
-// Lanczos vector kernels (FP64 scalars; vectors in T: FP64, or FP32 in the
-// mixed-precision setups whose operator is FP32 anyway).
-// w -= a v (a from device memory); block partials of ||w||^2
-template <class T>
-__global__ void __launch_bounds__(kRedThreads) k_axpy_norm(T* __restrict__ w, const T* __restrict__ v,
-                                                           const double* __restrict__ a_dev, i64 n,
-                                                           double* __restrict__ part) {
-  const double a = *a_dev;
+// Device scalars of a level's Lanczos run (alpha_j and beta_j follow the host's
+// order in an array of their own).
+struct LzScalars {
+  double inv;       // 1 / beta of the last step (the start vector's norm before the first)
+  double last;      // that beta
+  int stop;         // breakdown: the later steps change nothing
+  int bad;          // first non-positive diagonal entry, or kLzGood
+  unsigned ticket;  // grid_sum's
+  int pad;
+};
+constexpr int kLzGood = 0x7fffffff;
+
+// Sum over the lanes that hold a row's result (lane 0 of each VS group).
+template <int VS, class T>
+__device__ __forceinline__ double rows_block_sum(T v) {
+  __shared__ double part[8];
+#pragma unroll
+  for (int o = VS; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = static_cast<double>(v);
+  __syncthreads();
   double s = 0.0;
-  if constexpr (std::is_same<T, float>::value) {
-    // FP32 vectors: FP32 update, each thread's squares summed in FP32 before
-    // the FP64 block sum (no per-element FP64 work)
-    const float af = static_cast<float>(a);
-    float sf = 0.0f;
-    for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads) {
-      const float wi = fmaf(-af, v[i], w[i]);
-      w[i] = wi;
-      sf = fmaf(wi, wi, sf);
-    }
-    s = static_cast<double>(sf);
-  } else {
-    for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads) {
-      const T wi = static_cast<T>(todbl(w[i]) - a * todbl(v[i]));
-      w[i] = wi;
-      s += todbl(wi) * todbl(wi);
-    }
-  }
-  s = block_sum<kRedThreads>(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += part[k];
+  return s;
 }
 
-// vp = v ; v = w / b ; tmp = s .* v
-// (b from device memory; nothing once the breakdown test has stopped the steps)
+// u_j and v_{j-1} of row i become w = S A v_j - beta_{j-1} v_{j-1} and v_j, from
+// y = (A t)_i; returns w_i v_i.
 template <class T>
-__global__ void k_lanczos_shift(T* __restrict__ v, T* __restrict__ vp, const T* __restrict__ w,
-                                const T* __restrict__ s, T* __restrict__ tmp,
-                                const double* __restrict__ b, const double* __restrict__ stop, i64 n) {
-  if (*stop != 0.0) return;
-  const double bj = *b;
-  if constexpr (std::is_same<T, float>::value) {
-    // FP32 vectors: FP32 arithmetic with 1 / beta formed once per block
-    __shared__ float inv_b;
-    if (threadIdx.x == 0) inv_b = static_cast<float>(1.0 / bj);
-    __syncthreads();
-    const float ib = inv_b;
-    for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-      vp[i] = v[i];
-      const float vi = w[i] * ib;
-      v[i] = vi;
-      tmp[i] = s[i] * vi;
-    }
-  } else {
-    for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-      vp[i] = v[i];
-      const T vi = static_cast<T>(todbl(w[i]) / bj);
-      v[i] = vi;
-      tmp[i] = static_cast<T>(todbl(s[i]) * todbl(vi));
-    }
+__device__ __forceinline__ T lz_row(T y, i64 i, const T* __restrict__ s, T* __restrict__ w, T* __restrict__ v, T inv,
+                                    T beta) {
+  const T vn = w[i] * inv;
+  const T wn = y * inv * s[i] - beta * v[i];
+  w[i] = wn;
+  v[i] = vn;
+  return wn * vn;
+}
+
+// matrix-free operators: y = A t is a vector
+template <class T>
+__global__ void __launch_bounds__(kRedThreads) k_lz_post(const T* __restrict__ y, const T* __restrict__ s,
+                                                         T* __restrict__ w, T* __restrict__ v, i64 n,
+                                                         double* __restrict__ alpha, double* __restrict__ part,
+                                                         LzScalars* __restrict__ sc) {
+  if (sc->stop) return;
+  const T inv = static_cast<T>(sc->inv), beta = static_cast<T>(sc->last);
+  T c = T(0);
+  for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads)
+    c += lz_row(y[i], i, s, w, v, inv, beta);
+  double total;
+  if (grid_sum(block_sum<kRedThreads>(static_cast<double>(c)), part, &sc->ticket, total)) *alpha = total;
+}
+
+// w -= alpha_j v, t = s w, beta_j = ||w|| and the reference's breakdown test
+// (beta_j <= 1e-12 |alpha_j|); ab = alpha_j, beta_j
+template <class T>
+__global__ void __launch_bounds__(kRedThreads) k_lz_norm(const T* __restrict__ s, T* __restrict__ w,
+                                                         const T* __restrict__ v, T* __restrict__ t, i64 n,
+                                                         double* __restrict__ ab, double* __restrict__ part,
+                                                         LzScalars* __restrict__ sc) {
+  if (sc->stop) return;
+  const T a = static_cast<T>(ab[0]);
+  T c = T(0);
+  for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads) {
+    const T wi = w[i] - a * v[i];
+    w[i] = wi;
+    t[i] = s[i] * wi;
+    c += wi * wi;
+  }
+  double total;
+  if (grid_sum(block_sum<kRedThreads>(static_cast<double>(c)), part, &sc->ticket, total)) {
+    const double b = sqrt(total);
+    ab[1] = b;
+    if (!(b > 1.0e-12 * fabs(ab[0]))) sc->stop = 1;
+    sc->last = b;
+    sc->inv = 1.0 / b;
   }
 }
 
-// v = start / nrm ; tmp = s .* v ; s = sqrt(dinv).  planes > 0: v, s and tmp in
-// component planes of that many nodes (three unknowns a node).
+// The scalars before a level's first kernel: norm = ||start||.
+__global__ void k_lz_reset(LzScalars* sc, double norm) {
+  sc->inv = 1.0 / norm;
+  sc->last = norm;
+  sc->stop = 0;
+  sc->bad = kLzGood;
+  sc->ticket = 0;
+}
+
+// Inverse diagonal of a level (1 / a_ii; the first entry that is not positive
+// is recorded) and the Lanczos start: s = sqrt(1 / a_ii), w = start, t = s w,
+// v = 0.  planes > 0: dinv32, s, w, t and v in component planes of that many
+// nodes (three unknowns a node).
 template <class T>
-__global__ void k_lanczos_start(const double* __restrict__ start, T* __restrict__ v,
-                                const double* __restrict__ nrm, const double* __restrict__ dinv,
-                                T* __restrict__ s, T* __restrict__ tmp, i64 n, i64 planes) {
-  const double inv = *nrm;
+__global__ void k_level_start(i32 n, const i32* __restrict__ node_of, const i32* __restrict__ first,
+                              const i32* __restrict__ self_slot, NodeView a, const i32* __restrict__ rowptr,
+                              const T* __restrict__ val, const double* __restrict__ start, double* __restrict__ dinv,
+                              float* __restrict__ dinv32, T* __restrict__ s, T* __restrict__ w, T* __restrict__ t,
+                              T* __restrict__ v, i64 planes, LzScalars* __restrict__ sc) {
   for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
+    const i32 I = node_of[i];
+    const i32 li = static_cast<i32>(i) - first[I];
+    const double d = static_cast<double>(val[rowptr[i] + a.off[self_slot[I]] + li]);
+    double inv = 0.0;
+    if (!(d > 0.0)) atomicMin(&sc->bad, static_cast<int>(i));
+    else inv = 1.0 / d;
+    dinv[i] = inv;
     const i64 o = planes > 0 ? (i % 3) * planes + i / 3 : i;
-    const double si = sqrt(dinv[i]);
-    s[o] = static_cast<T>(si);
-    const double vi = todbl(static_cast<T>(start[i])) / inv;
-    v[o] = static_cast<T>(vi);
-    tmp[o] = static_cast<T>(todbl(static_cast<T>(si)) * todbl(static_cast<T>(vi)));
+    if (dinv32) dinv32[o] = static_cast<float>(inv);
+    const T si = static_cast<T>(sqrt(inv)), wi = static_cast<T>(start[i]);
+    s[o] = si;
+    w[o] = wi;
+    t[o] = si * wi;
+    v[o] = T(0);
   }
+}
+
+// Chebyshev coefficients and the prolongator's damping into device memory.
+struct ChebValues {
+  double v[64];
+  double omega;
+  int count;
+};
+__global__ void k_set_cheb(const __grid_constant__ ChebValues c, double* __restrict__ c64, float* __restrict__ c32,
+                           float* __restrict__ omega) {
+  const int k = threadIdx.x;
+  if (k < c.count) {
+    c64[k] = c.v[k];
+    c32[k] = static_cast<float>(c.v[k]);
+  }
+  if (k == 0) *omega = static_cast<float>(c.omega);
 }
 
 // ---------------------------------------------------------------------------
 // Setup numerics over node-level patterns
 // ---------------------------------------------------------------------------
-// 1 / diagonal; status 1 when a diagonal is not positive
-template <class TV>
-__global__ void k_inv_diag(i32 n, const i32* __restrict__ node_of, const i32* __restrict__ first,
-                           const i32* __restrict__ self_slot, NodeView a, const i32* __restrict__ rowptr,
-                           const TV* __restrict__ val, double* __restrict__ dinv, int* __restrict__ bad) {
-  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-    const i32 I = node_of[i];
-    const i32 li = static_cast<i32>(i) - first[I];
-    const double d = static_cast<double>(val[rowptr[i] + a.off[self_slot[I]] + li]);
-    if (!(d > 0.0)) {
-      atomicMin(bad, static_cast<int>(i));
-      dinv[i] = 0.0;
-    } else {
-      dinv[i] = 1.0 / d;
-    }
-  }
-}
-
 // Block sums of squares per node-level slot (strength of connection,
 // src/fem/Multigrid.cpp:460-513): rows of the row node in order, then the
 // slot's columns in order.

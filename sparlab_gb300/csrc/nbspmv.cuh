@@ -144,6 +144,26 @@ __global__ void __launch_bounds__(256) k_rows_cheb_first(i32 rows, const i32* __
   }
 }
 
+// A Lanczos step's operator rows (kernels.cuh): w and v of the step and alpha_j
+template <int VS, int B, class T>
+__global__ void __launch_bounds__(256) k_lz_rows(i32 rows, const i32* __restrict__ node_of, NodeView pat,
+                                                 const i32* __restrict__ rowptr, const i32* __restrict__ col,
+                                                 const T* __restrict__ val, const T* __restrict__ t,
+                                                 const T* __restrict__ s, T* __restrict__ w, T* __restrict__ v,
+                                                 double* __restrict__ alpha, double* __restrict__ part,
+                                                 LzScalars* __restrict__ sc) {
+  if (sc->stop) return;
+  const i64 q = blockIdx.x * (i64)blockDim.x + threadIdx.x;
+  const i32 row = static_cast<i32>(q / VS);
+  const int lane = static_cast<int>(q % VS);
+  const bool valid = row < rows;
+  const T y = rows_dot<VS, B, T, T>(row, lane, valid, node_of, pat, rowptr, col, val, t);
+  T c = T(0);
+  if (valid && lane == 0) c = lz_row(y, row, s, w, v, static_cast<T>(sc->inv), static_cast<T>(sc->last));
+  double total;
+  if (grid_sum(rows_block_sum<VS>(c), part, &sc->ticket, total)) *alpha = total;
+}
+
 // Double-float operator (mixed precision's CG operator): values stored as
 // hi + lo float pairs, x as (hi, lo) pairs, products and sums in
 // double-float arithmetic on the FP32 pipes, y in FP64.  About 2^-44 relative
