@@ -490,6 +490,31 @@ GpuAmg::GpuAmg(const AmgOptions& o) : opt(o) {
   mf_status.alloc(1);
   SIMP_CUDA(cudaMemset(mf_status.p, 0, sizeof(int)));
   main_.stream = stream;
+  init_reductions(main_);
+}
+
+void GpuAmg::init_reductions(SolveWork& w) {
+  w.part.alloc(kRedBlocks);
+  w.scal.alloc((sizeof(PcgScalars) + 7) / 8);
+  w.scal.zero(w.stream);
+  w.post.alloc(1);
+  *w.post.p = PcgPost{};
+}
+
+// Polls the post: a copy and a synchronisation of the stream cost several
+// microseconds an iteration.  The stream's state is looked at now and then,
+// so a failed launch ends the wait.
+void GpuAmg::wait_post(SolveWork& w) {
+  const volatile unsigned* seq = &w.post.p->seq;
+  for (unsigned spin = 1; *seq != w.seq; ++spin) {
+    if (spin % 64 == 0) std::this_thread::yield();
+    if (spin % 4096 != 0) continue;
+    const cudaError_t e = cudaStreamQuery(w.stream);
+    if (e == cudaErrorNotReady) continue;
+    SIMP_CUDA(e);
+    if (*seq != w.seq) throw Error(kCudaError, "a reduction ended without posting its sum");
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
 }
 
 void GpuAmg::check_mf_status(cudaStream_t s) {
@@ -526,6 +551,7 @@ SolveWork& GpuAmg::work(int k) {
     std::unique_ptr<SolveWork> w(new SolveWork());
     SIMP_CUDA(cudaStreamCreate(&w->stream));
     w->own_stream = true;
+    init_reductions(*w);
     extra_.push_back(std::move(w));
   }
   return *extra_[static_cast<size_t>(k - 1)];
@@ -552,10 +578,11 @@ void GpuAmg::ensure(SolveWork& w) {
     }
   }
   const size_t n0 = levels.empty() ? 0 : static_cast<size_t>(levels.front()->n);
-  w.part.alloc(kRedBlocks);
-  w.scal.alloc(16);
-  for (DBuf<double>* b : {&w.pr, &w.pz, &w.pp, &w.pq}) b->alloc(n0);
-  if (mixed()) w.xsplit.alloc(n0);
+  for (DBuf<double>* b : {&w.pp, &w.pq}) b->alloc(n0);
+  if (mixed()) {
+    w.pr.alloc(n0);
+    w.xsplit.alloc(n0);
+  }
 }
 
 Level& GpuAmg::level0() {
@@ -564,18 +591,10 @@ Level& GpuAmg::level0() {
 }
 
 double GpuAmg::dot(SolveWork& w, const double* a, const double* b, i64 n) {
-  // the context's own workspace uses the context's reduction buffers, so a
-  // dot works before ensure() (setup's Lanczos)
-  double* pt = &w == &main_ ? part.p : w.part.p;
-  double* sc = &w == &main_ ? scal.p : w.scal.p;
-  k_dot_partial<double, double><<<kRedBlocks, kRedThreads, 0, w.stream>>>(a, b, n, pt);
+  k_dot<<<red_blocks(n), kRedThreads, 0, w.stream>>>(a, b, n, w.part.p, w.scalars(), w.post.p, ++w.seq);
   SIMP_CHECK_LAUNCH();
-  k_reduce_final<<<1, kRedThreads, 0, w.stream>>>(pt, kRedBlocks, sc, 0);
-  SIMP_CHECK_LAUNCH();
-  double h = 0.0;
-  SIMP_CUDA(cudaMemcpyAsync(&h, sc, sizeof(double), cudaMemcpyDeviceToHost, w.stream));
-  SIMP_CUDA(cudaStreamSynchronize(w.stream));
-  return h;
+  wait_post(w);
+  return w.post.p->rr;
 }
 
 void GpuAmg::make_ops(size_t l) {
@@ -1583,36 +1602,48 @@ void GpuAmg::apply(SolveWork& w, const double* r, double* z) {
 // Preconditioned CG on A x = b (FP64 operator and vectors) from the guess in
 // x; `restarts` follows the reference's true-residual restarts.  Stops when
 // the recursive residual reaches `target` or the iteration `budget` is spent.
-// PCG iteration k > 1, second half of k - 1 and first half of k: z = M r,
-// beta, p = z + beta p (and p's double-float split), then q = A p, alpha,
-// x += alpha p, r -= alpha q, ||r||^2 -- no host value in between.
+// PCG iteration k, second half of k - 1 and first half of k: z = M r, beta, p =
+// z + beta p (and p's double-float split), then q = A p, alpha, x += alpha p, r
+// -= alpha q, ||r||^2 -- no host value in between.  r's FP32 copy is already
+// the V-cycle's right-hand side (k_pcg_begin, k_pcg_update).
 void GpuAmg::pcg_tail(SolveWork& w, float2* psplit) {
-  const i32 n = levels.front()->n;
+  const i32 n = levels.front()->n, planes = plane_nodes();
   const cudaStream_t stream = w.stream;
-  PcgScalars* sc = reinterpret_cast<PcgScalars*>(w.scal.p + 8);
-  apply(w, w.pr.p, w.pz.p);
-  k_dot_partial<double, double><<<kRedBlocks, kRedThreads, 0, stream>>>(w.pr.p, w.pz.p, n, w.part.p);
-  SIMP_CHECK_LAUNCH();
-  k_pcg_beta<<<1, kRedThreads, 0, stream>>>(w.part.p, kRedBlocks, sc);
-  SIMP_CHECK_LAUNCH();
-  k_pcg_direction<<<grid_for(n, 256), 256, 0, stream>>>(w.pp.p, w.pz.p, n, sc, psplit,
-                                                         mf_cg() ? w.p32.p : nullptr);
-  SIMP_CHECK_LAUNCH();
+  auto direction = [&](const auto* z) {
+    k_pcg_rz<<<red_blocks(n), kRedThreads, 0, stream>>>(residual(w), z, n, planes, w.part.p, w.scalars());
+    SIMP_CHECK_LAUNCH();
+    k_pcg_direction<<<grid_for(n, 256), 256, 0, stream>>>(w.pp.p, z, n, planes, w.scalars(), psplit,
+                                                           mf_cg() ? w.p32.p : nullptr);
+    SIMP_CHECK_LAUNCH();
+  };
+  if (mixed()) {
+    cycle<float>(w, 0);
+    direction(w.lv.front().x32.p);
+  } else {
+    cycle<double>(w, 0);
+    direction(w.lv.front().x64.p);
+  }
 }
 
 void GpuAmg::pcg_head(SolveWork& w, double* x, bool split_ready, bool op_done) {
   const i32 n = levels.front()->n;
   const cudaStream_t stream = w.stream;
-  PcgScalars* sc = reinterpret_cast<PcgScalars*>(w.scal.p + 8);
   if (!op_done) cg_op(w, w.pp.p, w.pq.p, split_ready);
-  k_dot_partial<double, double><<<kRedBlocks, kRedThreads, 0, stream>>>(w.pp.p, w.pq.p, n, w.part.p);
+  k_pcg_pq<<<red_blocks(n), kRedThreads, 0, stream>>>(w.pp.p, w.pq.p, n, w.part.p, w.scalars());
   SIMP_CHECK_LAUNCH();
-  k_pcg_alpha<<<1, kRedThreads, 0, stream>>>(w.part.p, kRedBlocks, sc);
+  k_pcg_update<<<red_blocks(n), kRedThreads, 0, stream>>>(x, residual(w), w.pp.p, w.pq.p, n, cycle_rhs32(w),
+                                                         plane_nodes(), w.part.p, w.scalars(), w.post.p);
   SIMP_CHECK_LAUNCH();
-  k_pcg_update<<<kRedBlocks, kRedThreads, 0, stream>>>(x, w.pr.p, w.pp.p, w.pq.p, n, sc, w.part.p);
+}
+
+double GpuAmg::pcg_begin(SolveWork& w, const double* b, const double* x) {
+  const i32 n = levels.front()->n;
+  op0(w, x, residual(w), b, false);
+  k_pcg_begin<<<red_blocks(n), kRedThreads, 0, w.stream>>>(residual(w), n, cycle_rhs32(w), plane_nodes(), w.part.p,
+                                                           w.scalars(), w.post.p, ++w.seq);
   SIMP_CHECK_LAUNCH();
-  k_reduce_final<<<1, kRedThreads, 0, stream>>>(w.part.p, kRedBlocks, &sc->rr, 0);
-  SIMP_CHECK_LAUNCH();
+  wait_post(w);
+  return std::sqrt(w.post.p->rr);
 }
 
 // pcg_tail + pcg_head as one graph launch: captured on the first use after a
@@ -1662,56 +1693,32 @@ GpuAmg::PcgResult GpuAmg::pcg(SolveWork& w, const double* b, double* x_out, doub
   w.px.alloc(static_cast<size_t>(n));
   double* x = w.px.p;
   SIMP_CUDA(cudaMemcpyAsync(x, x_out, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
-  DBuf<double>& pr = w.pr;
-  DBuf<double>& pz = w.pz;
-  DBuf<double>& pp = w.pp;
   PcgResult res;
-  PcgScalars* sc = reinterpret_cast<PcgScalars*>(w.scal.p + 8);
-  static_assert(sizeof(PcgScalars) <= 8 * sizeof(double), "scalar block");
-  auto op = [&](const double* in, double* out, const double* rhs) { op0(w, in, out, rhs, false); };
-  auto dot = [&](const double* a, const double* c, i64 m) { return this->dot(w, a, c, m); };
-  auto apply = [&](const double* r, double* z) { this->apply(w, r, z); };
   // mixed: the direction update also writes p's double-float split (or,
   // with the matrix-free CG operator, its FP32 copy)
   float2* psplit = psplit_of(w);
   if (mf_cg()) w.p32.alloc(static_cast<size_t>(n));
-  const bool p_copy = psplit != nullptr || mf_cg();
-  bool p_split = false;
   int total = 0;
   bool rec_conv = false;
   double best = std::numeric_limits<double>::max();
   // the FP32 products of the matrix-free CG operator make each restart a
   // step of iterative refinement on the FP64 true residual: allow more
   const int rounds = restarts ? (mf_cg() ? 12 : 3) : 1;
+  double rnorm = pcg_begin(w, b, x);
   for (int restart = 0; restart < rounds; ++restart) {
-    op(x, pr.p, b);
-    double rnorm = std::sqrt(dot(pr.p, pr.p, n));
     res.relres = rnorm / bnorm;
     if (rnorm <= target) { res.converged = true; break; }
-    apply(pr.p, pz.p);
-    SIMP_CUDA(cudaMemcpyAsync(pp.p, pz.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
-    const double rz = dot(pr.p, pz.p, n);
-    {
-      PcgScalars h{};
-      h.rz = rz;
-      SIMP_CUDA(cudaMemcpyAsync(sc, &h, sizeof(h), cudaMemcpyHostToDevice, stream));
-    }
     bool conv = false;
-    p_split = false;
-    bool first = true;
     while (total < budget) {
-      if (first) {
-        pcg_head(w, x, false);
-        first = false;
-      } else if (opt.graphs) {
+      ++w.seq;
+      if (opt.graphs) {
         pcg_body(w, x, psplit);
       } else {
         pcg_tail(w, psplit);
-        pcg_head(w, x, p_split);
+        pcg_head(w, x, psplit != nullptr || mf_cg());
       }
-      PcgScalars h{};
-      SIMP_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, stream));
-      SIMP_CUDA(cudaStreamSynchronize(stream));
+      wait_post(w);
+      const PcgPost& h = *w.post.p;
       if (h.status != 0) {
         std::ostringstream os;
         os << "preconditioned CG broke down at iteration " << total + 1 << " (p^T A p = " << h.pq
@@ -1722,16 +1729,16 @@ GpuAmg::PcgResult GpuAmg::pcg(SolveWork& w, const double* b, double* x_out, doub
       ++total;
       rnorm = std::sqrt(h.rr);
       if (rnorm <= target) { conv = true; break; }
-      p_split = p_copy;
     }
     if (!restarts) {
       res.converged = conv;
       res.relres = rnorm / bnorm;
       break;
     }
-    op(x, pr.p, b);
-    res.relres = std::sqrt(dot(pr.p, pr.p, n)) / bnorm;
-    if (res.relres * bnorm <= target) { res.converged = true; break; }
+    // the true residual, which a restart begins from
+    rnorm = pcg_begin(w, b, x);
+    res.relres = rnorm / bnorm;
+    if (rnorm <= target) { res.converged = true; break; }
     if (!conv) break;
     rec_conv = true;
     if (!(res.relres < 0.5 * best)) break;
@@ -1913,7 +1920,7 @@ struct TogetherGraph {
           a.pcg_tail(w, ps);
           if (fused[i]) return;
           a.pcg_head(w, w.px.p, ps != nullptr || a.mf_cg());
-          k_loop_test<<<1, 1, 0, w.stream>>>(reinterpret_cast<const PcgScalars*>(w.scal.p + 8), w.loop.p,
+          k_loop_test<<<1, 1, 0, w.stream>>>(w.scalars(), w.loop.p,
                                              w.loopd.p, flags.p + i, static_cast<int>(n));
           SIMP_CHECK_LAUNCH();
         });
@@ -1961,7 +1968,7 @@ struct TogetherGraph {
             SolveWork& w = *members[i].second;
             add_conditional(g, op, second[i], w, kernels[i], [&] {
               a.pcg_head(w, w.px.p, true, true);
-              k_loop_test<<<1, 1, 0, w.stream>>>(reinterpret_cast<const PcgScalars*>(w.scal.p + 8), w.loop.p,
+              k_loop_test<<<1, 1, 0, w.stream>>>(w.scalars(), w.loop.p,
                                                  w.loopd.p, flags.p + i, static_cast<int>(n));
               SIMP_CHECK_LAUNCH();
             });
@@ -2035,7 +2042,7 @@ void each_task(size_t n, F&& fn) {
 
 std::vector<GpuAmg::TaskResult> GpuAmg::solve_together(std::vector<SolveTask>& tasks) {
   struct St {
-    double bnorm = 0, target = 0, best = std::numeric_limits<double>::max();
+    double bnorm = 0, target = 0, rnorm = 0, best = std::numeric_limits<double>::max();
     int total = 0, round = 0, rounds = 3;
     bool done = false, rec_conv = false, conv = false, looping = false, ran = false;
   };
@@ -2100,35 +2107,16 @@ std::vector<GpuAmg::TaskResult> GpuAmg::solve_together(std::vector<SolveTask>& t
       SolveWork& w = *tasks[i].w;
       const i32 nn = a.levels.front()->n;
       try {
-        a.op0(w, w.px.p, w.pr.p, tasks[i].b, false);
-        const double rnorm = std::sqrt(a.dot(w, w.pr.p, w.pr.p, nn));
-        out[i].r.relres = rnorm / s.bnorm;
-        if (rnorm <= s.target) {
+        if (s.round == 0) s.rnorm = a.pcg_begin(w, tasks[i].b, w.px.p);  // (later rounds: the last one's end)
+        out[i].r.relres = s.rnorm / s.bnorm;
+        if (s.rnorm <= s.target) {
           out[i].r.converged = true;
           finish(i);
           return;
         }
-        a.apply(w, w.pr.p, w.pz.p);
-        SIMP_CUDA(cudaMemcpyAsync(w.pp.p, w.pz.p, sizeof(double) * nn, cudaMemcpyDeviceToDevice, w.stream));
-        const double rz = a.dot(w, w.pr.p, w.pz.p, nn);
-        PcgScalars* sc = reinterpret_cast<PcgScalars*>(w.scal.p + 8);
-        PcgScalars h{};
-        h.rz = rz;
-        SIMP_CUDA(cudaMemcpyAsync(sc, &h, sizeof(h), cudaMemcpyHostToDevice, w.stream));
         s.conv = false;
         s.ran = true;
-        if (s.total < a.opt.maxit) {
-          a.pcg_head(w, w.px.p, false);
-          SIMP_CUDA(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, w.stream));
-          SIMP_CUDA(cudaStreamSynchronize(w.stream));
-          if (h.status != 0) {
-            breakdown(i, h);
-            return;
-          }
-          ++s.total;
-          if (std::sqrt(h.rr) <= s.target) s.conv = true;
-          else if (s.total < a.opt.maxit) s.looping = true;
-        }
+        s.looping = s.total < a.opt.maxit;
         if (s.looping) {
           const int hl[4] = {1, s.total, a.opt.maxit, 0};
           const double ht[2] = {s.target, 0.0};
@@ -2184,9 +2172,10 @@ std::vector<GpuAmg::TaskResult> GpuAmg::solve_together(std::vector<SolveTask>& t
         SolveWork& w = *tasks[i].w;
         PcgScalars h{};
         int hl[4] = {0, 0, 0, 0};
-        SIMP_CUDA(cudaMemcpyAsync(&h, w.scal.p + 8, sizeof(h), cudaMemcpyDeviceToHost, w.stream));
+        SIMP_CUDA(cudaMemcpyAsync(&h, w.scal.p, sizeof(h), cudaMemcpyDeviceToHost, w.stream));
         SIMP_CUDA(cudaMemcpyAsync(hl, w.loop.p, sizeof(hl), cudaMemcpyDeviceToHost, w.stream));
         SIMP_CUDA(cudaStreamSynchronize(w.stream));
+        w.seq = h.seq;  // the bodies' posts were not awaited
         if (h.status != 0) {
           st[i].total = hl[1] - 1;  // the iteration that broke down is not counted
           breakdown(i, h);
@@ -2204,9 +2193,9 @@ std::vector<GpuAmg::TaskResult> GpuAmg::solve_together(std::vector<SolveTask>& t
       SolveWork& w = *tasks[i].w;
       const i32 nn = a.levels.front()->n;
       try {
-        a.op0(w, w.px.p, w.pr.p, tasks[i].b, false);
-        out[i].r.relres = std::sqrt(a.dot(w, w.pr.p, w.pr.p, nn)) / s.bnorm;
-        if (out[i].r.relres * s.bnorm <= s.target) {
+        s.rnorm = a.pcg_begin(w, tasks[i].b, w.px.p);
+        out[i].r.relres = s.rnorm / s.bnorm;
+        if (s.rnorm <= s.target) {
           out[i].r.converged = true;
           finish(i);
           return;

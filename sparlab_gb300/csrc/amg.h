@@ -183,7 +183,9 @@ struct SolveWork {
   cudaStream_t stream = 0;
   bool own_stream = false;
   std::vector<LevelWork> lv;
-  DBuf<double> part, scal, pr, pz, pp, pq;
+  DBuf<double> part, scal, pr, pp, pq;  // pr: the residual in mixed precision (FP64: level 0's b64)
+  PinnedBuf<PcgPost> post;              // the scalars a solve posts to the host
+  unsigned seq = 0;                     // number of its last awaited post
   DBuf<float2> xsplit;  // op0's input as (hi, lo) pairs (mixed mode)
   DBuf<float> p32;      // the CG direction in FP32 (matrix-free CG operator)
   // PCG iteration body (V-cycle, direction, operator, update) captured as a
@@ -200,6 +202,7 @@ struct SolveWork {
   SolveWork(const SolveWork&) = delete;
   SolveWork& operator=(const SolveWork&) = delete;
   ~SolveWork();
+  PcgScalars* scalars() const { return reinterpret_cast<PcgScalars*>(scal.p); }
 };
 
 struct AmgStats {
@@ -346,6 +349,17 @@ class GpuAmg {
   void pcg_tail(SolveWork& w, float2* psplit);
   // op_done: q = A p is already in w.pq (a fused multi-RHS launch)
   void pcg_head(SolveWork& w, double* x, bool split_ready, bool op_done = false);
+  // r = b - A x in w's residual, ||r|| (posted and awaited), and the scalars of
+  // a new CG run from it
+  double pcg_begin(SolveWork& w, const double* b, const double* x);
+  // reduction scratch, scalars and the posted values of a workspace
+  void init_reductions(SolveWork& w);
+  // waits until the post numbered w.seq has arrived
+  void wait_post(SolveWork& w);
+  // the residual: the V-cycle's level-0 right-hand side itself in FP64
+  double* residual(SolveWork& w) { return mixed() ? w.pr.p : w.lv.front().b64.p; }
+  float* cycle_rhs32(SolveWork& w) { return mixed() ? w.lv.front().b32.p : nullptr; }
+  i32 plane_nodes() const { return mf.planes ? mf.free_nodes : 0; }
   // q = A0 p of several workspaces of this hierarchy (mixed precision, p's
   // split in each xsplit) as one fused multi-RHS kernel node of g after
   // deps; a workspace whose loop flag is clear is skipped

@@ -118,6 +118,27 @@ struct PinnedBuf {
   }
 };
 
+// Scalars of a PCG solve in device memory (kernels.cuh).
+struct PcgScalars {
+  double rz;        // r^T z of the current direction
+  double pq;        // p^T A p
+  double alpha, beta;
+  double rr;        // ||r||^2 after the update
+  int status;       // 0 ok, 2 breakdown (p^T A p <= 0 or non-finite)
+  int fresh;        // 1: the next direction starts a CG run (beta = 0)
+  unsigned ticket;  // grid_sum's
+  unsigned seq;     // posts to the host so far
+};
+
+// What the host reads after an iteration, in page-locked memory that the last
+// block of the update writes: the host polls seq instead of copying and
+// synchronising.
+struct PcgPost {
+  double rr, pq;
+  int status;
+  unsigned seq;
+};
+
 // Raises a kernel's dynamic shared-memory limit to at least `bytes` and never
 // lowers it: the limit is one value per kernel, shared by every host thread,
 // so a thread that set a smaller value could make another thread's larger

@@ -214,74 +214,87 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce_final(const double* __re
 }
 
 // ---------------------------------------------------------------------------
-// PCG scalars and vector updates (FP64 CG scalars in device memory)
+// PCG scalars and vector updates (FP64 CG scalars in device memory).  Each
+// reduction is one launch (grid_sum); a CG iteration is the V-cycle and five
+// launches: r^T z with beta, the direction, the operator, p^T q with alpha, the
+// update.  z is read where the V-cycle left it (its level-0 iterate, FP32 in
+// mixed precision) and the update writes the next V-cycle's right-hand side,
+// so no pass converts or copies between them.
 // ---------------------------------------------------------------------------
-struct PcgScalars {
-  double rz;       // r^T z of the current direction
-  double pq;       // p^T A p
-  double alpha, beta;
-  double rr;       // ||r||^2 after the update
-  double rz_new;
-  int status;      // 0 ok, 2 breakdown (p^T A p <= 0 or non-finite)
-  int pad;
-};
+__device__ __forceinline__ void post_to_host(const PcgScalars* sc, PcgPost* host) {
+  host->rr = sc->rr;
+  host->pq = sc->pq;
+  host->status = sc->status;
+  __threadfence_system();
+  *reinterpret_cast<volatile unsigned*>(&host->seq) = sc->seq;
+}
 
-__global__ void __launch_bounds__(kRedThreads) k_pcg_alpha(const double* __restrict__ part, int m,
-                                                           PcgScalars* sc) {
+// Place of unknown i in a vector in component planes of `nodes` nodes, three
+// unknowns a node.
+__device__ __forceinline__ i32 plane_of(i32 i, i32 nodes) { return i % 3 * nodes + i / 3; }
+
+// out[0] = a^T b, to the host
+__global__ void __launch_bounds__(kRedThreads) k_dot(const double* __restrict__ a, const double* __restrict__ b, i64 n,
+                                                     double* __restrict__ part, PcgScalars* sc, PcgPost* host,
+                                                     unsigned seq) {
   double s = 0.0;
-  for (int i = threadIdx.x; i < m; i += kRedThreads) s += part[i];
-  s = block_sum<kRedThreads>(s);
-  if (threadIdx.x == 0) {
-    sc->pq = s;
-    if (!(s > 0.0) || !isfinite(s)) {
-      sc->status = 2;
-      sc->alpha = 0.0;
-    } else {
-      sc->alpha = sc->rz / s;
-    }
+  for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads) s += a[i] * b[i];
+  double total;
+  if (grid_sum(block_sum<kRedThreads>(s), part, &sc->ticket, total)) {
+    sc->rr = total;
+    sc->seq = seq;
+    post_to_host(sc, host);
   }
 }
 
-// rz_new = sum(part); beta = rz_new / rz; rz = rz_new
-__global__ void __launch_bounds__(kRedThreads) k_pcg_beta(const double* __restrict__ part, int m,
-                                                          PcgScalars* sc) {
+// ||r||^2 to the host, the V-cycle's FP32 right-hand side (planes > 0: in
+// component planes), and the scalars of a new CG run
+__global__ void __launch_bounds__(kRedThreads) k_pcg_begin(const double* __restrict__ r, i32 n, float* __restrict__ b32,
+                                                           i32 planes, double* __restrict__ part, PcgScalars* sc,
+                                                           PcgPost* host, unsigned seq) {
   double s = 0.0;
-  for (int i = threadIdx.x; i < m; i += kRedThreads) s += part[i];
-  s = block_sum<kRedThreads>(s);
-  if (threadIdx.x == 0) {
-    sc->rz_new = s;
-    sc->beta = s / sc->rz;
-    sc->rz = s;
-  }
-}
-
-// x += alpha p ; r -= alpha q ; partial ||r||^2
-__global__ void __launch_bounds__(kRedThreads) k_pcg_update(double* __restrict__ x, double* __restrict__ r,
-                                                            const double* __restrict__ p,
-                                                            const double* __restrict__ q, i64 n,
-                                                            const PcgScalars* __restrict__ sc,
-                                                            double* __restrict__ part) {
-  const double alpha = sc->alpha;
-  double s = 0.0;
-  for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads) {
-    x[i] += alpha * p[i];
-    const double ri = r[i] - alpha * q[i];
-    r[i] = ri;
+  for (i32 i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) {
+    const double ri = r[i];
     s += ri * ri;
+    if (b32) b32[planes > 0 ? plane_of(i, planes) : i] = static_cast<float>(ri);
   }
-  s = block_sum<kRedThreads>(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
+  double total;
+  if (grid_sum(block_sum<kRedThreads>(s), part, &sc->ticket, total)) {
+    sc->rr = total;
+    sc->rz = 0.0;
+    sc->status = 0;
+    sc->fresh = 1;
+    sc->seq = seq;
+    post_to_host(sc, host);
+  }
 }
 
-// p = z + beta p; with ps, also its double-float split (the next operator
-// application's input in mixed precision); with p32, its FP32 copy (the
-// input of the matrix-free CG operator)
-__global__ void k_pcg_direction(double* __restrict__ p, const double* __restrict__ z, i64 n,
-                                const PcgScalars* __restrict__ sc, float2* __restrict__ ps,
-                                float* __restrict__ p32) {
+// r^T z; beta = r^T z / the last one (0 for the first direction)
+template <class TZ>
+__global__ void __launch_bounds__(kRedThreads) k_pcg_rz(const double* __restrict__ r, const TZ* __restrict__ z, i32 n,
+                                                        i32 planes, double* __restrict__ part, PcgScalars* sc) {
+  double s = 0.0;
+  for (i32 i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads)
+    s += r[i] * static_cast<double>(z[planes > 0 ? plane_of(i, planes) : i]);
+  double total;
+  if (grid_sum(block_sum<kRedThreads>(s), part, &sc->ticket, total)) {
+    sc->beta = sc->fresh ? 0.0 : total / sc->rz;
+    sc->rz = total;
+    sc->fresh = 0;
+  }
+}
+
+// p = z + beta p (p = z where a run starts); with ps, also its double-float
+// split (the operator's input in mixed precision); with p32, its FP32 copy
+// (the input of the matrix-free CG operator)
+template <class TZ>
+__global__ void __launch_bounds__(256) k_pcg_direction(double* __restrict__ p, const TZ* __restrict__ z, i32 n,
+                                                       i32 planes, const PcgScalars* __restrict__ sc,
+                                                       float2* __restrict__ ps, float* __restrict__ p32) {
   const double beta = sc->beta;
-  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-    const double v = z[i] + beta * p[i];
+  for (i32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double v = static_cast<double>(z[planes > 0 ? plane_of(i, planes) : i]);
+    if (beta != 0.0) v += beta * p[i];
     p[i] = v;
     if (ps) {
       float h, l;
@@ -289,6 +302,47 @@ __global__ void k_pcg_direction(double* __restrict__ p, const double* __restrict
       ps[i] = make_float2(h, l);
     }
     if (p32) p32[i] = __double2float_rn(v);
+  }
+}
+
+// p^T q and alpha
+__global__ void __launch_bounds__(kRedThreads) k_pcg_pq(const double* __restrict__ p, const double* __restrict__ q,
+                                                        i32 n, double* __restrict__ part, PcgScalars* sc) {
+  double s = 0.0;
+  for (i32 i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) s += p[i] * q[i];
+  double total;
+  if (grid_sum(block_sum<kRedThreads>(s), part, &sc->ticket, total)) {
+    sc->pq = total;
+    if (!(total > 0.0) || !isfinite(total)) {
+      sc->status = 2;
+      sc->alpha = 0.0;
+    } else {
+      sc->alpha = sc->rz / total;
+    }
+  }
+}
+
+// x += alpha p ; r -= alpha q ; ||r||^2 to the host ; r's FP32 copy as the next
+// V-cycle's right-hand side
+__global__ void __launch_bounds__(kRedThreads) k_pcg_update(double* __restrict__ x, double* __restrict__ r,
+                                                            const double* __restrict__ p,
+                                                            const double* __restrict__ q, i32 n,
+                                                            float* __restrict__ b32, i32 planes,
+                                                            double* __restrict__ part, PcgScalars* sc, PcgPost* host) {
+  const double alpha = sc->alpha;
+  double s = 0.0;
+  for (i32 i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) {
+    x[i] += alpha * p[i];
+    const double ri = r[i] - alpha * q[i];
+    r[i] = ri;
+    if (b32) b32[planes > 0 ? plane_of(i, planes) : i] = static_cast<float>(ri);
+    s += ri * ri;
+  }
+  double total;
+  if (grid_sum(block_sum<kRedThreads>(s), part, &sc->ticket, total)) {
+    sc->rr = total;
+    sc->seq += 1u;
+    post_to_host(sc, host);
   }
 }
 
