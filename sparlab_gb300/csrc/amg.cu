@@ -1303,24 +1303,12 @@ void GpuAmg::coarse_factorize() {
   dense_.alloc(nn);
   swept_.alloc(nn);
   piv_.alloc(n);
-  panel_.alloc(2 * static_cast<size_t>(n) * kNB + kNB * kNB);
-  double* pu = panel_.p;
-  double* pv = pu + static_cast<size_t>(n) * kNB;
-  double* pp = pv + static_cast<size_t>(n) * kNB;
+  panel_.alloc(sweep_panel_size(n));
   SIMP_CUDA(cudaMemsetAsync(swept_.p, 0, nn * sizeof(double), stream));
   k_dense_from_csr<<<grid_for(n, 128), 128, 0, stream>>>(n, lv.a.ptr.p, lv.a.col.p, lv.a.v64.p, swept_.p);
   SIMP_CHECK_LAUNCH();
   SIMP_CUDA(cudaMemsetAsync(dstatus.p, 0, sizeof(int), stream));
-  const int nt = (n + kNB - 1) / kNB;
-  const dim3 tiles(nt, nt);
-  for (int k0 = 0; k0 < n; k0 += kNB) {
-    const int kb = std::min(kNB, n - k0);
-    k_sweep_pivot<false><<<(n + kSweepRows - 1) / kSweepRows, 256, 0, stream>>>(swept_.p, n, k0, kb, pu, pv,
-                                                                                 pp, piv_.p, dstatus.p);
-    SIMP_CHECK_LAUNCH();
-    k_sweep_update<<<tiles, 256, 0, stream>>>(swept_.p, n, k0, kb, pu, pv, pp);
-    SIMP_CHECK_LAUNCH();
-  }
+  dense_sweep<false>(swept_.p, n, panel_.p, piv_.p, dstatus.p, stream);
   int status = 0;
   SIMP_CUDA(cudaMemcpyAsync(&status, dstatus.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
   const std::vector<double> piv = piv_.to_host(stream);
@@ -1338,7 +1326,8 @@ void GpuAmg::coarse_factorize() {
        << "level, so the model is under-constrained: too few supports, or a part connected to nothing";
     throw Error(kUnderConstrained, os.str());
   }
-  k_sweep_finish<<<tiles, 256, 0, stream>>>(swept_.p, dense_.p, n);
+  const int nt = (n + kNB - 1) / kNB;
+  k_sweep_finish<<<dim3(nt, nt), 256, 0, stream>>>(swept_.p, dense_.p, n);
   SIMP_CHECK_LAUNCH();
 }
 

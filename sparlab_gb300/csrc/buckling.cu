@@ -275,31 +275,20 @@ struct ShiftedInverse {
     const size_t nn = static_cast<size_t>(n) * n;
     swept.alloc(nn);
     inv.alloc(nn);
-    panel.alloc(2 * static_cast<size_t>(n) * kNB + kNB * kNB);
+    panel.alloc(sweep_panel_size(n));
     piv.alloc(static_cast<size_t>(n));
     status.alloc(1);
   }
 
   int factor(const Level& l0, const double* kval, const double* gval, double sig) {
     const size_t nn = static_cast<size_t>(n) * n;
-    double* pu = panel.p;
-    double* pv = pu + static_cast<size_t>(n) * kNB;
-    double* pp = pv + static_cast<size_t>(n) * kNB;
     SIMP_CUDA(cudaMemsetAsync(swept.p, 0, nn * sizeof(double), s));
     SIMP_CUDA(cudaMemsetAsync(status.p, 0, sizeof(int), s));
     k_dense_shifted<<<grid_for(n, 128), 128, 0, s>>>(n, l0.a.ptr.p, l0.a.col.p, kval, gval, sig, swept.p);
     SIMP_CHECK_LAUNCH();
+    dense_sweep<true>(swept.p, n, panel.p, piv.p, status.p, s);
     const int nt = (n + kNB - 1) / kNB;
-    const dim3 tiles(nt, nt);
-    for (int k0 = 0; k0 < n; k0 += kNB) {
-      const int kb = std::min(kNB, n - k0);
-      k_sweep_pivot<true><<<(n + kSweepRows - 1) / kSweepRows, 256, 0, s>>>(swept.p, n, k0, kb, pu, pv, pp,
-                                                                            piv.p, status.p);
-      SIMP_CHECK_LAUNCH();
-      k_sweep_update<<<tiles, 256, 0, s>>>(swept.p, n, k0, kb, pu, pv, pp);
-      SIMP_CHECK_LAUNCH();
-    }
-    k_sweep_finish<<<tiles, 256, 0, s>>>(swept.p, inv.p, n);
+    k_sweep_finish<<<dim3(nt, nt), 256, 0, s>>>(swept.p, inv.p, n);
     SIMP_CHECK_LAUNCH();
     int bad = 0;
     SIMP_CUDA(cudaMemcpyAsync(&bad, status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
