@@ -484,8 +484,6 @@ double seconds_since(std::chrono::steady_clock::time_point t0) {
 // own kernels on device pointers it passes in) stays ordered with it.
 GpuAmg::GpuAmg(const AmgOptions& o) : opt(o) {
   SIMP_CUDA(cudaStreamCreate(&stream));
-  part.alloc(kRedBlocks);
-  scal.alloc(16);
   dstatus.alloc(4);
   mf_status.alloc(1);
   SIMP_CUDA(cudaMemset(mf_status.p, 0, sizeof(int)));
@@ -504,18 +502,19 @@ void GpuAmg::init_reductions(SolveWork& w) {
 // Polls the post: a copy and a synchronisation of the stream cost several
 // microseconds an iteration.  The stream's state is looked at now and then,
 // so a failed launch ends the wait.
-void GpuAmg::wait_post(SolveWork& w) {
-  const volatile unsigned* seq = &w.post.p->seq;
-  for (unsigned spin = 1; *seq != w.seq; ++spin) {
+void wait_for_post(const volatile unsigned* seq, unsigned value, cudaStream_t stream) {
+  for (unsigned spin = 1; *seq != value; ++spin) {
     if (spin % 64 == 0) std::this_thread::yield();
     if (spin % 4096 != 0) continue;
-    const cudaError_t e = cudaStreamQuery(w.stream);
+    const cudaError_t e = cudaStreamQuery(stream);
     if (e == cudaErrorNotReady) continue;
     SIMP_CUDA(e);
-    if (*seq != w.seq) throw Error(kCudaError, "a reduction ended without posting its sum");
+    if (*seq != value) throw Error(kCudaError, "a reduction ended without posting its sum");
   }
   std::atomic_thread_fence(std::memory_order_acquire);
 }
+
+void GpuAmg::wait_post(SolveWork& w) { wait_for_post(&w.post.p->seq, w.seq, w.stream); }
 
 void GpuAmg::check_mf_status(cudaStream_t s) {
   if (!mf.tensor) return;

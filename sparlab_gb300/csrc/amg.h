@@ -312,7 +312,6 @@ class GpuAmg {
   static std::vector<TaskResult> solve_together(std::vector<SolveTask>& tasks);
   double dot(SolveWork& w, const double* a, const double* b, i64 n);
 
-  DBuf<double> part, scal;  // reductions of setup and of callers on the context stream
   DBuf<int> dstatus;
   DBuf<int> mf_status;  // the tensor-core matrix-free kernel's wait status
   // throws when a tensor-core matrix-free launch on this stream reported a

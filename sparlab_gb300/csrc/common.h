@@ -139,6 +139,17 @@ struct PcgPost {
   unsigned seq;
 };
 
+// Sums that a kernel's last block leaves in page-locked memory for the host.
+struct SumPost {
+  static constexpr int kValues = 7;
+  double v[kValues];
+  unsigned seq;
+};
+
+// Polls a post until it shows `value`.  A fault of the stream, or its end
+// without the post, becomes an error.
+void wait_for_post(const volatile unsigned* seq, unsigned value, cudaStream_t stream);
+
 // Raises a kernel's dynamic shared-memory limit to at least `bytes` and never
 // lowers it: the limit is one value per kernel, shared by every host thread,
 // so a thread that set a smaller value could make another thread's larger

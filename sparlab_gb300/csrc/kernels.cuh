@@ -131,9 +131,10 @@ __device__ __forceinline__ double block_sum(double v) {
 // stores its partial and takes a ticket, and the last one adds the partials in
 // order, so the value does not depend on which block that is.  True in that
 // block's thread 0, with the total; the ticket is back at zero for the next
-// launch.
+// launch.  `also` runs in all threads of that block.
+template <class Last>
 __device__ __forceinline__ bool grid_sum(double block, double* __restrict__ part, unsigned* __restrict__ ticket,
-                                         double& total) {
+                                         double& total, Last also) {
   __shared__ int last;
   if (threadIdx.x == 0) {
     part[blockIdx.x] = block;
@@ -146,10 +147,79 @@ __device__ __forceinline__ bool grid_sum(double block, double* __restrict__ part
   double s = 0.0;
   for (unsigned i = threadIdx.x; i < gridDim.x; i += 256) s += __ldcg(part + i);
   s = block_sum<256>(s);
+  also();
   if (threadIdx.x != 0) return false;
   *ticket = 0u;
   total = s;
   return true;
+}
+
+__device__ __forceinline__ bool grid_sum(double block, double* __restrict__ part, unsigned* __restrict__ ticket,
+                                         double& total) {
+  return grid_sum(block, part, ticket, total, [] {});
+}
+
+// Sums of K values of every thread over the grid, in one launch and in the
+// order in which grid_sum would add each of them: the
+// lanes of a warp halve the set of values that they still hold at each step
+// (K = 7 costs 9 additions where 7 separate sums cost 35; the FP64 pipe takes
+// 16 clocks for each), every block stores its K partials, and a warp of the
+// last block adds up a row of partials and stores the total in page-locked
+// memory that the host polls.  Blocks of 256 threads; part holds K * gridDim.x.
+template <int D>  // K = 2^D - 1 values and a zero
+__device__ __forceinline__ void grid_sums_to_host(double (&s)[1 << D], double* __restrict__ part,
+                                                  unsigned* __restrict__ ticket, SumPost* host, unsigned seq) {
+  constexpr int P = 1 << D, K = P - 1;
+  static_assert(K <= SumPost::kValues, "");
+  __shared__ double warp_part[P][9];
+  __shared__ int last;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+  for (int step = 0; step < D; ++step) {
+    const int half = P >> (step + 1), off = 16 >> step;
+    const bool up = (l & off) != 0;
+#pragma unroll
+    for (int i = 0; i < P / 2; ++i) {
+      if (i >= half) continue;
+      const double give = up ? s[i] : s[i + half], keep = up ? s[i + half] : s[i];
+      s[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+    }
+  }
+#pragma unroll
+  for (int off = 16 >> D; off > 0; off >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], off);
+  if ((l & ((32 >> D) - 1)) == 0) warp_part[l >> (5 - D)][w] = s[0];
+  auto of_warps = [](const double* v) { return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7])); };
+  __syncthreads();
+  const unsigned nb = gridDim.x;
+  if (threadIdx.x < K) {
+    part[threadIdx.x * nb + blockIdx.x] = of_warps(warp_part[threadIdx.x]);
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == nb - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int k = w; k < K; k += 8) {
+    double v[8] = {};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (q * 32u >= nb) continue;
+      double t = 0.0;
+      for (unsigned i = q * 32u + l; i < nb; i += 256) t += __ldcg(part + k * nb + i);
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      v[q] = t;
+    }
+    if (l == 0) {
+      host->v[k] = of_warps(v);
+      __threadfence_system();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *ticket = 0u;
+    *reinterpret_cast<volatile unsigned*>(&host->seq) = seq;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -179,38 +249,6 @@ __global__ void k_from_planes(const A* __restrict__ a, B* __restrict__ b, i64 no
   for (i64 I = blockIdx.x * (i64)blockDim.x + threadIdx.x; I < nodes; I += (i64)gridDim.x * blockDim.x)
 #pragma unroll
     for (int k = 0; k < 3; ++k) b[3 * I + k] = static_cast<B>(a[k * nodes + I]);
-}
-
-// ---------------------------------------------------------------------------
-// deterministic two-stage reductions
-// ---------------------------------------------------------------------------
-template <class TA, class TB>
-__global__ void __launch_bounds__(kRedThreads) k_dot_partial(const TA* __restrict__ a,
-                                                             const TB* __restrict__ b, i64 n,
-                                                             double* __restrict__ part) {
-  double s = 0.0;
-  if constexpr (std::is_same<TA, float>::value && std::is_same<TB, float>::value) {
-    // FP32 vectors (the reuse setups' Lanczos): each thread's products summed
-    // in FP32 before the FP64 block sum (no per-element FP64 work)
-    float sf = 0.0f;
-    for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads)
-      sf = fmaf(a[i], b[i], sf);
-    s = static_cast<double>(sf);
-  } else {
-    for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads)
-      s += todbl(a[i]) * todbl(b[i]);
-  }
-  s = block_sum<kRedThreads>(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-// out = sum(part[0..m)) ; optional sqrt
-__global__ void __launch_bounds__(kRedThreads) k_reduce_final(const double* __restrict__ part, int m,
-                                                              double* __restrict__ out, int take_sqrt) {
-  double s = 0.0;
-  for (int i = threadIdx.x; i < m; i += kRedThreads) s += part[i];
-  s = block_sum<kRedThreads>(s);
-  if (threadIdx.x == 0) *out = take_sqrt ? sqrt(s) : s;
 }
 
 // ---------------------------------------------------------------------------

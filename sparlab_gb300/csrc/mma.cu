@@ -393,19 +393,7 @@ OcStep GpuProblem::mma_update(bool apply, double* xnew_host) {
   st.bisections = total;
   st.converged = true;
   st.volume = 0.0;
-  // max |x' - x| and the grey level of the evaluated density
-  k_change_gray<<<kRedBlocks, kRedThreads, 0, s>>>(ne, m_x.p, x.p, rho.p, opart.p, opart.p + kRedBlocks);
-  SIMP_CHECK_LAUNCH();
-  std::vector<double> hp(2 * kRedBlocks);
-  SIMP_CUDA(cudaMemcpyAsync(hp.data(), opart.p, sizeof(double) * 2 * kRedBlocks, cudaMemcpyDeviceToHost, s));
-  SIMP_CUDA(cudaStreamSynchronize(s));
-  double mc = 0.0, gs = 0.0;
-  for (int k = 0; k < kRedBlocks; ++k) {
-    mc = std::max(mc, hp[k]);
-    gs += hp[kRedBlocks + k];
-  }
-  st.max_change = mc;
-  gray = 4.0 * gs / static_cast<double>(ne);
+  change_and_gray(st, m_x.p);
   if (xnew_host) {
     m_x.download(xnew_host, nn, s);
     SIMP_CUDA(cudaStreamSynchronize(s));

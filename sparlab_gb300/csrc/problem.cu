@@ -298,7 +298,10 @@ void GpuProblem::build() {
   se.alloc(ne_s);
   tmp.alloc(ne_s);
   opart.alloc(static_cast<size_t>(std::max(2, kOcSpec)) * kRedBlocks);
-  ovol.alloc(kOcSpec);
+  oc_post.alloc(1);
+  oc_post.p->seq = 0;
+  oc_ticket.alloc(1);
+  oc_ticket.zero(amg.stream);
   // loads restricted to the free DOFs
   std::vector<double> bh(static_cast<size_t>(nfree) * d.nloads);
   for (int l = 0; l < d.nloads; ++l)
@@ -696,12 +699,7 @@ Evaluation GpuProblem::evaluate_finish(const std::vector<GpuAmg::PcgResult>& res
     filter_adjoint(dc_dphys.p, dc_dx.p);
   }
   // volume of the physical density
-  k_dot_partial<double, double><<<kRedBlocks, kRedThreads, 0, s>>>(rho.p, vols.p, ne, amg.part.p);
-  SIMP_CHECK_LAUNCH();
-  k_reduce_final<<<1, kRedThreads, 0, s>>>(amg.part.p, kRedBlocks, amg.scal.p + 4, 0);
-  SIMP_CHECK_LAUNCH();
-  SIMP_CUDA(cudaMemcpyAsync(&ev.volume, amg.scal.p + 4, sizeof(double), cudaMemcpyDeviceToHost, s));
-  SIMP_CUDA(cudaStreamSynchronize(s));
+  ev.volume = amg.dot(amg.work(0), rho.p, vols.p, ne);
   ev.volume_fraction = ev.volume / domain_volume;
   if (d.robust && d.eta_override <= 0.0) {
     // robust_volumes (TopologyOptimizer.cpp:61-80): the blueprint's volume,
@@ -798,6 +796,17 @@ void GpuProblem::update_robust_target() {
     dilated_target = d.vf * domain_volume * ev.volume_dilated / ev.volume_intermediate;
 }
 
+// max |x' - x| and the grey level of the evaluated density
+void GpuProblem::change_and_gray(OcStep& st, const double* candidate) {
+  cudaStream_t s = amg.stream;
+  k_change_gray<<<grid_for(ne, kRedThreads, kRedBlocks), kRedThreads, 0, s>>>(ne, candidate, x.p, rho.p, opart.p,
+                                                                             oc_ticket.p, oc_post.p, ++oc_seq);
+  SIMP_CHECK_LAUNCH();
+  wait_for_post(&oc_post.p->seq, oc_seq, s);
+  st.max_change = oc_post.p->v[0];
+  gray = 4.0 * oc_post.p->v[1] / static_cast<double>(ne);
+}
+
 OcStep GpuProblem::oc_update(bool apply, double* xnew_host) {
   if (!evaluated) throw Error(kBadInput, "oc_update needs gradients: call evaluate first");
   cudaStream_t s = amg.stream;
@@ -814,27 +823,80 @@ OcStep GpuProblem::oc_update(bool apply, double* xnew_host) {
                                                 d.damping, oc_g.p, oc_lo.p, oc_hi.p);
   SIMP_CHECK_LAUNCH();
   auto factor = [&](double lam) { return d.damping == 0.5 ? 1.0 / std::sqrt(lam) : std::pow(lam, -d.damping); };
+  const int blocks = grid_for(ne, kRedThreads, kRedBlocks);
+  SumPost* post = oc_post.p;
+  auto wait = [&] {
+    SIMP_CHECK_LAUNCH();
+    wait_for_post(&post->seq, oc_seq, s);
+  };
   auto volume_of = [&](double lam) {
     if (d.projection) {
       // the projected volume is not linear in the design: candidate, then a
       // filter + projection pass (volume_of_design of run_oc)
       k_oc_apply<<<grid_for(ne, 256), 256, 0, s>>>(ne, oc_g.p, oc_lo.p, oc_hi.p, factor(lam), xnew.p);
       SIMP_CHECK_LAUNCH();
-      k_filter_volume_projected<<<kRedBlocks, kRedThreads, 0, s>>>(
-          grid_of(d), static_cast<const Stencil*>(stencil_d), hw.p, ne, xnew.p, vols.p, beta, d.volume_eta(), part);
+      k_filter_volume_projected<<<blocks, kRedThreads, 0, s>>>(grid_of(d), static_cast<const Stencil*>(stencil_d),
+                                                               hw.p, ne, xnew.p, vols.p, beta, d.volume_eta(), part,
+                                                               oc_ticket.p, post, ++oc_seq);
     } else {
-      k_oc_volume<<<kRedBlocks, kRedThreads, 0, s>>>(ne, oc_g.p, oc_lo.p, oc_hi.p, dv_dx.p, factor(lam), part);
+      OcFactors f{};
+      f.t[0] = factor(lam);
+      k_oc_volume<1><<<blocks, kRedThreads, 0, s>>>(ne, oc_g.p, oc_lo.p, oc_hi.p, dv_dx.p, f, part, oc_ticket.p, post,
+                                                    ++oc_seq);
     }
-    SIMP_CHECK_LAUNCH();
-    k_reduce_final<<<1, kRedThreads, 0, s>>>(part, kRedBlocks, amg.scal.p + 5, 0);
-    SIMP_CHECK_LAUNCH();
-    double v = 0.0;
-    SIMP_CUDA(cudaMemcpyAsync(&v, amg.scal.p + 5, sizeof(double), cudaMemcpyDeviceToHost, s));
-    SIMP_CUDA(cudaStreamSynchronize(s));
-    return v;
+    wait();
+    return post->v[0];
+  };
+  auto volumes_of = [&](const double* lam, int count, double* v) {
+    OcFactors f{};
+    for (int k = 0; k < kOcSpec; ++k) f.t[k] = factor(lam[std::min(k, count - 1)]);
+    k_oc_volume<kOcDepth><<<blocks, kRedThreads, 0, s>>>(ne, oc_g.p, oc_lo.p, oc_hi.p, dv_dx.p, f, part, oc_ticket.p,
+                                                         post, ++oc_seq);
+    wait();
+    std::copy(post->v, post->v + count, v);
+  };
+  // The bisection of optimality_criteria_update, evaluated speculatively:
+  // one pass computes the volumes of the bracket's midpoint and of the
+  // midpoints either outcome leads to (a depth-3 tree of 7 multipliers), and
+  // the host walks the tree with the sequential rules, so the multipliers,
+  // volumes and stopping point are the one-by-one loop's.  It saves host
+  // round trips where they dominate; on large grids, where a pass's 7 FP64
+  // candidates cost more than the round trips, the depth is 1 (one midpoint
+  // per pass, the plain loop).
+  const int depth = (d.projection || ne > (1 << 20)) ? 1 : kOcDepth;
+  // the midpoints of a tree of n nodes below [tl[0], th[0]]
+  double tl[kOcSpec], th[kOcSpec], mids[kOcSpec], mid_vols[kOcSpec];
+  auto midpoints = [&](int n) {
+    for (int k = 0; k < n; ++k) {
+      mids[k] = std::sqrt(tl[k] * th[k]);
+      if (2 * k + 2 < n) {
+        tl[2 * k + 1] = mids[k];  // vol > target: lo = mid
+        th[2 * k + 1] = th[k];
+        tl[2 * k + 2] = tl[k];    // else: hi = mid
+        th[2 * k + 2] = mids[k];
+      }
+    }
   };
   double lo = 1.0e-12, hi = 1.0e12;
-  double vlo = volume_of(lo), vhi = volume_of(hi);
+  double vlo, vhi;
+  int ready = 0;  // nodes of the first tree whose volumes came with the bracket's
+  if (depth > 1) {
+    ready = kOcSpec / 2;
+    double lam[kOcSpec], v[kOcSpec];
+    tl[0] = lo;
+    th[0] = hi;
+    midpoints(ready);
+    lam[0] = lo;
+    lam[1] = hi;
+    std::copy(mids, mids + ready, lam + 2);
+    volumes_of(lam, ready + 2, v);
+    vlo = v[0];
+    vhi = v[1];
+    std::copy(v + 2, v + 2 + ready, mid_vols);
+  } else {
+    vlo = volume_of(lo);
+    vhi = volume_of(hi);
+  }
   int widen = 0;
   while (vlo < target && widen < 60) {
     lo *= 1.0e-3;
@@ -861,48 +923,21 @@ OcStep GpuProblem::oc_update(bool apply, double* xnew_host) {
        << " m^3: the move-limited box yields volumes in [" << vhi << ", " << vlo << "] m^3";
     throw Error(kMaxIter, os.str());
   }
+  if (widen > 0) ready = 0;
   double vol = corner ? st.volume : vlo;
-  // The bisection of optimality_criteria_update, evaluated speculatively:
-  // one pass computes the volumes of the bracket's midpoint and of the
-  // midpoints either outcome leads to (a depth-3 tree of 7 multipliers), and
-  // the host walks the tree with the sequential rules, so the multipliers,
-  // volumes and stopping point are the one-by-one loop's.  It saves host
-  // round trips where they dominate; on large grids, where a pass's 7 FP64
-  // candidates cost more than the round trips, the depth is 1 (one midpoint
-  // per pass, the plain loop).
-  const int depth = (d.projection || ne > (1 << 20)) ? 1 : 3;
   int it = 0;
   bool done = corner;
   while (!done && it < 200) {
-    double tl[kOcSpec], th[kOcSpec], mids[kOcSpec], vols[kOcSpec];
-    const int nodes = (1 << depth) - 1;
+    const int nodes = ready > 0 ? ready : (1 << depth) - 1;
     tl[0] = lo;
     th[0] = hi;
-    for (int k = 0; k < nodes; ++k) {
-      mids[k] = std::sqrt(tl[k] * th[k]);
-      if (2 * k + 2 < nodes) {
-        tl[2 * k + 1] = mids[k];  // vol > target: lo = mid
-        th[2 * k + 1] = th[k];
-        tl[2 * k + 2] = tl[k];    // else: hi = mid
-        th[2 * k + 2] = mids[k];
-      }
-    }
-    if (nodes == 1) {
-      vols[0] = volume_of(mids[0]);
-    } else {
-      OcFactors f{};
-      for (int k = 0; k < nodes; ++k) f.t[k] = factor(mids[k]);
-      k_oc_volume_multi<kOcSpec><<<kRedBlocks, kRedThreads, 0, s>>>(ne, oc_g.p, oc_lo.p, oc_hi.p, dv_dx.p, f,
-                                                                    part);
-      SIMP_CHECK_LAUNCH();
-      k_reduce_rows<<<nodes, kRedThreads, 0, s>>>(part, kRedBlocks, ovol.p);
-      SIMP_CHECK_LAUNCH();
-      SIMP_CUDA(cudaMemcpyAsync(vols, ovol.p, sizeof(double) * nodes, cudaMemcpyDeviceToHost, s));
-      SIMP_CUDA(cudaStreamSynchronize(s));
-    }
+    midpoints(nodes);
+    if (ready > 0) ready = 0;
+    else if (nodes == 1) mid_vols[0] = volume_of(mids[0]);
+    else volumes_of(mids, nodes, mid_vols);
     for (int k = 0; k < nodes && !done;) {
       const double mid = mids[k];
-      vol = vols[k];
+      vol = mid_vols[k];
       st.bisections = ++it;
       st.lambda = mid;
       if (std::abs(vol - target) <= 1.0e-10 * target) {
@@ -928,19 +963,7 @@ OcStep GpuProblem::oc_update(bool apply, double* xnew_host) {
                                               xnew.p);
   SIMP_CHECK_LAUNCH();
   st.volume = vol;
-  // max |x' - x| and the grey level of the evaluated density
-  k_change_gray<<<kRedBlocks, kRedThreads, 0, s>>>(ne, xnew.p, x.p, rho.p, part, part + kRedBlocks);
-  SIMP_CHECK_LAUNCH();
-  std::vector<double> hp(2 * kRedBlocks);
-  SIMP_CUDA(cudaMemcpyAsync(hp.data(), part, sizeof(double) * 2 * kRedBlocks, cudaMemcpyDeviceToHost, s));
-  SIMP_CUDA(cudaStreamSynchronize(s));
-  double mc = 0.0, gs = 0.0;
-  for (int k = 0; k < kRedBlocks; ++k) {
-    mc = std::max(mc, hp[k]);
-    gs += hp[kRedBlocks + k];
-  }
-  st.max_change = mc;
-  gray = 4.0 * gs / static_cast<double>(ne);
+  change_and_gray(st, xnew.p);
   if (xnew_host) {
     xnew.download(xnew_host, static_cast<size_t>(ne), s);
     SIMP_CUDA(cudaStreamSynchronize(s));

@@ -351,14 +351,16 @@ __global__ void k_mul(i64 ne, const double* __restrict__ a, const double* __rest
     out[e] = a[e] * b[e];
 }
 
-// Projected filtered volume of a candidate design: block partials of
-// sum_e v_e rho_bar(clamp((H x)_e)) (the OC trial volume with projection on).
+// Projected filtered volume of a candidate design, sum_e v_e
+// rho_bar(clamp((H x)_e)) (the OC trial volume with projection on).
 __global__ void __launch_bounds__(kRedThreads) k_filter_volume_projected(GridView g, const Stencil* __restrict__ st,
                                                                          const double* __restrict__ w, i64 ne,
                                                                          const double* __restrict__ x,
                                                                          const double* __restrict__ volumes,
                                                                          double beta, double eta,
-                                                                         double* __restrict__ part) {
+                                                                         double* __restrict__ part,
+                                                                         unsigned* ticket, SumPost* host,
+                                                                         unsigned seq) {
   double vs = 0.0;
   for (i64 e = blockIdx.x * (i64)kRedThreads + threadIdx.x; e < ne; e += (i64)gridDim.x * kRedThreads) {
     const i32 ex = static_cast<i32>(e % g.nx), ey = static_cast<i32>((e / g.nx) % g.ny),
@@ -374,8 +376,8 @@ __global__ void __launch_bounds__(kRedThreads) k_filter_volume_projected(GridVie
     double dp;
     vs += project_one(s, beta, eta, dp) * volumes[e];
   }
-  vs = block_sum<kRedThreads>(vs);
-  if (threadIdx.x == 0) part[blockIdx.x] = vs;
+  double sum[2] = {vs, 0.0};
+  grid_sums_to_host<1>(sum, part, ticket, host, seq);
 }
 
 // Per OC update (src/topopt/OptimalityCriteria.cpp:14-38 restated for a
@@ -398,59 +400,36 @@ __global__ void k_oc_prepare(i64 ne, const double* __restrict__ x, const double*
   }
 }
 
-// Filtered volume of the candidate of multiplier lam (t = lam^-eta): the
-// volume sum_e v_e (H x')_e equals c^T x' with c = H^T v (dv_dx), so a trial
-// needs no filter pass.  Block partials of sum_e c_e clamp(g_e t, lo_e, hi_e).
-__global__ void __launch_bounds__(kRedThreads) k_oc_volume(i64 ne, const double* __restrict__ g,
-                                                           const double* __restrict__ lo,
-                                                           const double* __restrict__ hi,
-                                                           const double* __restrict__ c, double t,
-                                                           double* __restrict__ part) {
-  double s = 0.0;
-  for (i64 e = blockIdx.x * (i64)kRedThreads + threadIdx.x; e < ne; e += (i64)gridDim.x * kRedThreads)
-    s += c[e] * fmin(fmax(g[e] * t, lo[e]), hi[e]);
-  s = block_sum<kRedThreads>(s);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-// The same block partials for K multipliers in one pass over the element
-// arrays (part[k * gridDim.x + block] for t[k]); each multiplier's sum is
-// formed exactly as k_oc_volume forms it.
-constexpr int kOcSpec = 7;  // multipliers of one speculative bisection pass
+// Filtered volumes of the candidates of K = 2^D - 1 multipliers lam (t =
+// lam^-eta) in one pass over the element arrays: sum_e v_e (H x')_e equals
+// c^T x' with c = H^T v (dv_dx), so a trial needs no filter pass, and is
+// sum_e c_e clamp(g_e t, lo_e, hi_e).  A multiplier's sum does not depend on
+// D.  Small grids are bound by the launch and the way back: a block for every
+// 256 elements and sums that end here and are posted, instead of 1024 blocks, a
+// second launch and a copy, took a 120 x 40 design pass from 3.01 to 2.47 ms;
+// large ones by the FP64 pipe (four operations a multiplier and element).
+constexpr int kOcDepth = 3;                     // of the tree of one speculative bisection pass
+constexpr int kOcSpec = (1 << kOcDepth) - 1;    // its multipliers
+static_assert(kOcSpec <= SumPost::kValues, "");
 struct OcFactors {
   double t[kOcSpec];
 };
 
-template <int K>
-__global__ void __launch_bounds__(kRedThreads) k_oc_volume_multi(i64 ne, const double* __restrict__ g,
-                                                                 const double* __restrict__ lo,
-                                                                 const double* __restrict__ hi,
-                                                                 const double* __restrict__ c, OcFactors f,
-                                                                 double* __restrict__ part) {
-  double s[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) s[k] = 0.0;
+template <int D>
+__global__ void __launch_bounds__(kRedThreads) k_oc_volume(i64 ne, const double* __restrict__ g,
+                                                           const double* __restrict__ lo,
+                                                           const double* __restrict__ hi,
+                                                           const double* __restrict__ c, OcFactors f,
+                                                           double* __restrict__ part, unsigned* ticket,
+                                                           SumPost* host, unsigned seq) {
+  constexpr int K = (1 << D) - 1;
+  double s[K + 1] = {};
   for (i64 e = blockIdx.x * (i64)kRedThreads + threadIdx.x; e < ne; e += (i64)gridDim.x * kRedThreads) {
     const double ge = g[e], le = lo[e], he = hi[e], ce = c[e];
 #pragma unroll
     for (int k = 0; k < K; ++k) s[k] += ce * fmin(fmax(ge * f.t[k], le), he);
   }
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const double v = block_sum<kRedThreads>(s[k]);
-    if (threadIdx.x == 0) part[k * gridDim.x + blockIdx.x] = v;
-  }
-}
-
-// out[k] = sum of part[k * m .. k * m + m), one block per k, each summed as
-// k_reduce_final sums (no square root)
-__global__ void __launch_bounds__(kRedThreads) k_reduce_rows(const double* __restrict__ part, int m,
-                                                             double* __restrict__ out) {
-  const double* pk = part + static_cast<i64>(blockIdx.x) * m;
-  double s = 0.0;
-  for (int i = threadIdx.x; i < m; i += kRedThreads) s += pk[i];
-  s = block_sum<kRedThreads>(s);
-  if (threadIdx.x == 0) out[blockIdx.x] = s;
+  grid_sums_to_host<D>(s, part, ticket, host, seq);
 }
 
 __global__ void k_oc_apply(i64 ne, const double* __restrict__ g, const double* __restrict__ lo,
@@ -459,27 +438,40 @@ __global__ void k_oc_apply(i64 ne, const double* __restrict__ g, const double* _
     xn[e] = fmin(fmax(g[e] * t, lo[e]), hi[e]);
 }
 
-// max |a - b| and sum rho (1 - rho) partials
+// max |a - b| and sum rho (1 - rho), posted to the host as v[0] and v[1]
+// (part holds 2 * gridDim.x; the last block adds the partials up in order)
 __global__ void __launch_bounds__(kRedThreads) k_change_gray(i64 ne, const double* __restrict__ a,
                                                              const double* __restrict__ b,
                                                              const double* __restrict__ rho,
-                                                             double* __restrict__ part_max,
-                                                             double* __restrict__ part_gray) {
+                                                             double* __restrict__ part, unsigned* ticket,
+                                                             SumPost* host, unsigned seq) {
+  __shared__ double wm[kRedThreads / 32];
+  auto block_max = [&](double m) {
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    for (int k = 0; k < kRedThreads / 32; ++k) m = fmax(m, wm[k]);
+    return m;
+  };
   double m = 0.0, gsum = 0.0;
   for (i64 e = blockIdx.x * (i64)kRedThreads + threadIdx.x; e < ne; e += (i64)gridDim.x * kRedThreads) {
     m = fmax(m, fabs(a[e] - b[e]));
-    if (rho) gsum += rho[e] * (1.0 - rho[e]);
+    gsum += rho[e] * (1.0 - rho[e]);
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __shared__ double wm[kRedThreads / 32];
-  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
-  gsum = block_sum<kRedThreads>(gsum);
-  if (threadIdx.x == 0) {
-    double mm = 0.0;
-    for (int k = 0; k < kRedThreads / 32; ++k) mm = fmax(mm, wm[k]);
-    part_max[blockIdx.x] = mm;
-    if (part_gray) part_gray[blockIdx.x] = gsum;
-  }
+  m = block_max(m);
+  if (threadIdx.x == 0) part[gridDim.x + blockIdx.x] = m;
+  double total;
+  // grid_sum's fence of thread 0 covers its maximum as well
+  const bool post = grid_sum(block_sum<kRedThreads>(gsum), part, ticket, total, [&] {
+    m = 0.0;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += kRedThreads) m = fmax(m, __ldcg(part + gridDim.x + i));
+    m = block_max(m);
+  });
+  if (!post) return;
+  host->v[0] = m;
+  host->v[1] = total;
+  __threadfence_system();
+  *reinterpret_cast<volatile unsigned*>(&host->seq) = seq;
 }
 
 __global__ void k_clamp01(i64 ne, double* __restrict__ x) {
