@@ -114,8 +114,8 @@ template <int MODE, class TV, class TX, class TA>
 void nb_apply(const NbOp& op, const TV* val, const TX* x, TX* y, const TX* b, cudaStream_t s) {
   with_shape<TA>(op, [&](auto vs, auto blk) {
     constexpr int VS = decltype(vs)::value, B = decltype(blk)::value;
-    k_rows_apply<VS, B, MODE, TV, TX, TA><<<rows_grid(op, VS), 256, 0, s>>>(
-        op.node_of, op.pat, op.rowptr, op.col, val, x, y, b, op.rows);
+    chain_launch(k_rows_apply<VS, B, MODE, TV, TX, TA>, rows_grid(op, VS), 256, 0, s,
+                 op.node_of, op.pat, op.rowptr, op.col, val, x, y, b, op.rows);
   });
   SIMP_CHECK_LAUNCH();
 }
@@ -125,8 +125,8 @@ void nb_cheb_step(const NbOp& op, const T* val, const T* d, const T* rin, T* r, 
                   const T* c12, int add_d, cudaStream_t s) {
   with_shape<T>(op, [&](auto vs, auto blk) {
     constexpr int VS = decltype(vs)::value, B = decltype(blk)::value;
-    k_rows_cheb_step<VS, B, T><<<rows_grid(op, VS), 256, 0, s>>>(
-        op.rows, op.node_of, op.pat, op.rowptr, op.col, val, d, rin, r, dn, x, dinv, c12, add_d);
+    chain_launch(k_rows_cheb_step<VS, B, T>, rows_grid(op, VS), 256, 0, s,
+                 op.rows, op.node_of, op.pat, op.rowptr, op.col, val, d, rin, r, dn, x, dinv, c12, add_d);
   });
   SIMP_CHECK_LAUNCH();
 }
@@ -136,8 +136,8 @@ void nb_cheb_first(const NbOp& op, const T* val, const T* x, const T* b, T* r, T
                    const T* inv_theta, cudaStream_t s) {
   with_shape<T>(op, [&](auto vs, auto blk) {
     constexpr int VS = decltype(vs)::value, B = decltype(blk)::value;
-    k_rows_cheb_first<VS, B, T><<<rows_grid(op, VS), 256, 0, s>>>(
-        op.rows, op.node_of, op.pat, op.rowptr, op.col, val, x, b, r, d, dinv, inv_theta);
+    chain_launch(k_rows_cheb_first<VS, B, T>, rows_grid(op, VS), 256, 0, s,
+                 op.rows, op.node_of, op.pat, op.rowptr, op.col, val, x, b, r, d, dinv, inv_theta);
   });
   SIMP_CHECK_LAUNCH();
 }
@@ -196,13 +196,13 @@ struct V<float> {
 // Level-0 vectors between node order and component planes, converting.
 template <class A, class B>
 void to_planes(const A* a, B* b, i64 nodes, cudaStream_t s) {
-  k_to_planes<A, B><<<grid_for(nodes, 256, 4096), 256, 0, s>>>(a, b, nodes);
+  chain_launch(k_to_planes<A, B>, grid_for(nodes, 256, 4096), 256, 0, s, a, b, nodes);
   SIMP_CHECK_LAUNCH();
 }
 
 template <class A, class B>
 void from_planes(const A* a, B* b, i64 nodes, cudaStream_t s) {
-  k_from_planes<A, B><<<grid_for(nodes, 256, 4096), 256, 0, s>>>(a, b, nodes);
+  chain_launch(k_from_planes<A, B>, grid_for(nodes, 256, 4096), 256, 0, s, a, b, nodes);
   SIMP_CHECK_LAUNCH();
 }
 
@@ -231,15 +231,15 @@ void mf3_64(const MfOp& mf, const double* x, double* y, const double* b, cudaStr
   const dim3 grid((mf.nnx + kTX - 1) / kTX, (mf.nny + kTY - 1) / kTY, (mf.nz + 1 + kTZ * kNZ - 1) / (kTZ * kNZ));
   KeF64 ke;
   std::copy(mf.ke64_host, mf.ke64_host + 24 * 24, ke.k);
-  k_mf3_tile64<MODE><<<grid, kTX * kTY * kTZ, 0, s>>>(mf_view(mf), mf.scale64, x, y, b, ke);
+  chain_launch(k_mf3_tile64<MODE>, grid, kTX * kTY * kTZ, 0, s, mf_view(mf), mf.scale64, x, y, b, ke);
   SIMP_CHECK_LAUNCH();
 }
 
 template <int MODE, int TX, int TY, int TZ>
 void mf3_shape(const MfOp& mf, const MfArgs& a, const KeF32& ke, cudaStream_t s, bool v4) {
   const dim3 grid((mf.nnx + TX - 1) / TX, (mf.nny + TY - 1) / TY, (mf.nz + 1 + TZ - 1) / TZ);
-  if (v4) k_mf3_tile<MODE, TX, TY, TZ, true><<<grid, TX * TY * TZ, 0, s>>>(mf_view(mf), a, ke);
-  else k_mf3_tile<MODE, TX, TY, TZ, false><<<grid, TX * TY * TZ, 0, s>>>(mf_view(mf), a, ke);
+  if (v4) chain_launch(k_mf3_tile<MODE, TX, TY, TZ, true>, grid, TX * TY * TZ, 0, s, mf_view(mf), a, ke);
+  else chain_launch(k_mf3_tile<MODE, TX, TY, TZ, false>, grid, TX * TY * TZ, 0, s, mf_view(mf), a, ke);
   SIMP_CHECK_LAUNCH();
 }
 
@@ -303,7 +303,7 @@ void mf3_par(const MfOp& mf, const MfArgs& a, cudaStream_t s) {
       for (int c = 0; c < 3; ++c) ke.k[l][r][c] = static_cast<float>(mf.kpar[l][r][c]);
   int layers = 0;
   const dim3 grid = par_grid(mf, kParRows, k_mf3_par<MODE, ParF32, kParRows>, &layers);
-  k_mf3_par<MODE, ParF32, kParRows><<<grid, 32 * (kParRows + 2), 0, s>>>(mf_view(mf), a, ke, layers);
+  chain_launch(k_mf3_par<MODE, ParF32, kParRows>, grid, 32 * (kParRows + 2), 0, s, mf_view(mf), a, ke, layers);
   SIMP_CHECK_LAUNCH();
 }
 
@@ -320,7 +320,7 @@ void mf3_df(const MfOp& mf, const float2* x, double* y, const double* b, cudaStr
   int layers = 0;
   const dim3 grid = par_grid(mf, kParRowsDf, k_mf3_par<MODE, ParDf, kParRowsDf>, &layers);
   const MfArgs64 a{x, y, b, mf.scale2};
-  k_mf3_par<MODE, ParDf, kParRowsDf><<<grid, 32 * (kParRowsDf + 2), 0, s>>>(mf_view(mf), a, ke, layers);
+  chain_launch(k_mf3_par<MODE, ParDf, kParRowsDf>, grid, 32 * (kParRowsDf + 2), 0, s, mf_view(mf), a, ke, layers);
   SIMP_CHECK_LAUNCH();
 }
 
@@ -361,7 +361,7 @@ void mf2(const MfOp& mf, const MfArgs& a, cudaStream_t s) {
   KeQ4 ke;
   std::copy(mf.ke_host, mf.ke_host + 8 * 8, ke.k);
   const unsigned grid = static_cast<unsigned>((mf.nnx + 31) / 32) * static_cast<unsigned>((mf.nny + 3) / 4);
-  k_mf2<MODE><<<grid, 128, 0, s>>>(mf_view(mf), a.x, a.y, a.b, a.r, a.dn, a.xs, a.dinv, a.coef, a.add_d, ke);
+  chain_launch(k_mf2<MODE>, grid, 128, 0, s, mf_view(mf), a.x, a.y, a.b, a.r, a.dn, a.xs, a.dinv, a.coef, a.add_d, ke);
   SIMP_CHECK_LAUNCH();
 }
 
@@ -434,7 +434,7 @@ void mf_restrict(const MfOp& mf, const Level& lv, const float* x, const float* b
   mf3<7>(mf, c, s);
   const i64 th = static_cast<i64>(lv.naggs) * 32;
   auto restrict_to = [&](auto kernel) {
-    kernel<<<grid_for(th, 256), 256, 0, s>>>(lv.naggs, lv.nnodes, lv.d_members_ptr.p, lv.d_members.p,
+    chain_launch(kernel, grid_for(th, 256), 256, 0, s, lv.naggs, lv.nnodes, lv.d_members_ptr.p, lv.d_members.p,
                                              lv.phat_ptr.p, lv.phat32.p, r, bc);
   };
   if (mf.planes) restrict_to(k_phat_restrict<6, true>);
@@ -444,7 +444,7 @@ void mf_restrict(const MfOp& mf, const Level& lv, const float* x, const float* b
 
 void mf_prolong(const MfOp& mf, const Level& lv, const float* xc, float* t, float* x, cudaStream_t s) {
   auto prolong = [&](auto kernel) {
-    kernel<<<grid_for(lv.n, 256), 256, 0, s>>>(lv.n, lv.d_agg.p, lv.phat_ptr.p, lv.phat32.p, xc, t);
+    chain_launch(kernel, grid_for(lv.n, 256), 256, 0, s, lv.n, lv.d_agg.p, lv.phat_ptr.p, lv.phat32.p, xc, t);
   };
   if (mf.planes) prolong(k_phat_prolong<6, true>);
   else prolong(k_phat_prolong<6, false>);
@@ -502,6 +502,8 @@ void GpuAmg::init_reductions(SolveWork& w) {
 // Polls the post: a copy and a synchronisation of the stream cost several
 // microseconds an iteration.  The stream's state is looked at now and then,
 // so a failed launch ends the wait.
+thread_local int t_chain_off = 0;
+
 void wait_for_post(const volatile unsigned* seq, unsigned value, cudaStream_t stream) {
   for (unsigned spin = 1; *seq != value; ++spin) {
     if (spin % 64 == 0) std::this_thread::yield();
@@ -677,10 +679,10 @@ void GpuAmg::df_apply_unroll(const float2* xsplit, double* y, const double* rhs,
     auto go = [&](auto ur) {
       constexpr int U = decltype(ur)::value;
       if (rhs)
-        k_rows_apply_df<VS, B, 1, U><<<grid, 256, 0, stream>>>(op.node_of, op.pat, op.rowptr, op.col, l0.a.v2.p,
+        chain_launch(k_rows_apply_df<VS, B, 1, U>, grid, 256, 0, stream, op.node_of, op.pat, op.rowptr, op.col, l0.a.v2.p,
                                                                xsplit, y, rhs, op.rows);
       else
-        k_rows_apply_df<VS, B, 0, U><<<grid, 256, 0, stream>>>(op.node_of, op.pat, op.rowptr, op.col, l0.a.v2.p,
+        chain_launch(k_rows_apply_df<VS, B, 0, U>, grid, 256, 0, stream, op.node_of, op.pat, op.rowptr, op.col, l0.a.v2.p,
                                                                xsplit, y, nullptr, op.rows);
     };
     if (unroll == 8) go(std::integral_constant<int, 8>{});
@@ -889,19 +891,19 @@ void GpuAmg::lanczos(size_t l, int m, double* ab) {
     if (matrix_free) {
       if constexpr (f32) {
         mf_apply(mf, t, lz_y_.p, stream);
-        k_lz_post<float><<<blocks, kRedThreads, 0, stream>>>(lz_y_.p, s, w, v, n, ab + 2 * j, pt, sc);
+        chain_launch(k_lz_post<float>, blocks, kRedThreads, 0, stream, lz_y_.p, s, w, v, n, ab + 2 * j, pt, sc);
         SIMP_CHECK_LAUNCH();
       }
     } else {
       with_shape<T>(lv.opA, [&](auto lanes, auto blk) {
         constexpr int VS = decltype(lanes)::value, B = decltype(blk)::value;
-        k_lz_rows<VS, B, T><<<rows_grid(lv.opA, VS), 256, 0, stream>>>(n, lv.opA.node_of, lv.opA.pat, lv.opA.rowptr,
+        chain_launch(k_lz_rows<VS, B, T>, rows_grid(lv.opA, VS), 256, 0, stream, n, lv.opA.node_of, lv.opA.pat, lv.opA.rowptr,
                                                                        lv.opA.col, values, t, s, w, v, ab + 2 * j, pt, sc);
       });
       SIMP_CHECK_LAUNCH();
     }
     if (j + 1 == m) break;  // beta of the last step is not used
-    k_lz_norm<T><<<blocks, kRedThreads, 0, stream>>>(s, w, v, t, n, ab + 2 * j, pt, sc);
+    chain_launch(k_lz_norm<T>, blocks, kRedThreads, 0, stream, s, w, v, t, n, ab + 2 * j, pt, sc);
     SIMP_CHECK_LAUNCH();
   }
 }
@@ -1326,7 +1328,7 @@ void GpuAmg::coarse_factorize() {
     throw Error(kUnderConstrained, os.str());
   }
   const int nt = (n + kNB - 1) / kNB;
-  k_sweep_finish<<<dim3(nt, nt), 256, 0, stream>>>(swept_.p, dense_.p, n);
+  chain_launch(k_sweep_finish, dim3(nt, nt), 256, 0, stream, swept_.p, dense_.p, n);
   SIMP_CHECK_LAUNCH();
 }
 
@@ -1336,7 +1338,7 @@ void GpuAmg::coarse_solve(SolveWork& w, size_t l) {
   const int n = nc_;
   const i64 th = static_cast<i64>(n) * 32;
   LevelWork& v = w.lv[l];
-  k_gemv<T, T><<<grid_for(th, 256), 256, 0, w.stream>>>(dense_.p, n, V<T>::b(v), V<T>::x(v));
+  chain_launch(k_gemv<T, T>, grid_for(th, 256), 256, 0, w.stream, dense_.p, n, V<T>::b(v), V<T>::x(v));
   SIMP_CHECK_LAUNCH();
 }
 
@@ -1510,7 +1512,7 @@ void GpuAmg::smooth(SolveWork& w, size_t l, bool zero_guess) {
   bool matrix_free = false;
   if constexpr (std::is_same<T, float>::value) matrix_free = l == 0 && mf.enabled;
   if (zero_guess) {
-    k_cheb_zero<T><<<grid_for(n, 256), 256, 0, stream>>>(n, b, dinv, d, x, V<T>::cheb(lv));
+    chain_launch(k_cheb_zero<T>, grid_for(n, 256), 256, 0, stream, n, b, dinv, d, x, V<T>::cheb(lv));
     SIMP_CHECK_LAUNCH();
   } else if (matrix_free) {
     if constexpr (std::is_same<T, float>::value)
@@ -1598,9 +1600,10 @@ void GpuAmg::pcg_tail(SolveWork& w, float2* psplit) {
   const i32 n = levels.front()->n, planes = plane_nodes();
   const cudaStream_t stream = w.stream;
   auto direction = [&](const auto* z) {
-    k_pcg_rz<<<red_blocks(n), kRedThreads, 0, stream>>>(residual(w), z, n, planes, w.part.p, w.scalars());
+    using TZ = std::remove_cv_t<std::remove_pointer_t<decltype(z)>>;
+    chain_launch(k_pcg_rz<TZ>, red_blocks(n), kRedThreads, 0, stream, residual(w), z, n, planes, w.part.p, w.scalars());
     SIMP_CHECK_LAUNCH();
-    k_pcg_direction<<<grid_for(n, 256), 256, 0, stream>>>(w.pp.p, z, n, planes, w.scalars(), psplit,
+    chain_launch(k_pcg_direction<TZ>, grid_for(n, 256), 256, 0, stream, w.pp.p, z, n, planes, w.scalars(), psplit,
                                                            mf_cg() ? w.p32.p : nullptr);
     SIMP_CHECK_LAUNCH();
   };
@@ -1617,9 +1620,9 @@ void GpuAmg::pcg_head(SolveWork& w, double* x, bool split_ready, bool op_done) {
   const i32 n = levels.front()->n;
   const cudaStream_t stream = w.stream;
   if (!op_done) cg_op(w, w.pp.p, w.pq.p, split_ready);
-  k_pcg_pq<<<red_blocks(n), kRedThreads, 0, stream>>>(w.pp.p, w.pq.p, n, w.part.p, w.scalars());
+  chain_launch(k_pcg_pq, red_blocks(n), kRedThreads, 0, stream, w.pp.p, w.pq.p, n, w.part.p, w.scalars());
   SIMP_CHECK_LAUNCH();
-  k_pcg_update<<<red_blocks(n), kRedThreads, 0, stream>>>(x, residual(w), w.pp.p, w.pq.p, n, cycle_rhs32(w),
+  chain_launch(k_pcg_update, red_blocks(n), kRedThreads, 0, stream, x, residual(w), w.pp.p, w.pq.p, n, cycle_rhs32(w),
                                                          plane_nodes(), w.part.p, w.scalars(), w.post.p);
   SIMP_CHECK_LAUNCH();
 }
@@ -1627,7 +1630,7 @@ void GpuAmg::pcg_head(SolveWork& w, double* x, bool split_ready, bool op_done) {
 double GpuAmg::pcg_begin(SolveWork& w, const double* b, const double* x) {
   const i32 n = levels.front()->n;
   op0(w, x, residual(w), b, false);
-  k_pcg_begin<<<red_blocks(n), kRedThreads, 0, w.stream>>>(residual(w), n, cycle_rhs32(w), plane_nodes(), w.part.p,
+  chain_launch(k_pcg_begin, red_blocks(n), kRedThreads, 0, w.stream, residual(w), n, cycle_rhs32(w), plane_nodes(), w.part.p,
                                                            w.scalars(), w.post.p, ++w.seq);
   SIMP_CHECK_LAUNCH();
   wait_post(w);
@@ -1830,6 +1833,7 @@ struct TogetherGraph {
     SIMP_CUDA(cudaStreamBeginCaptureToGraph(w.stream, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                             cudaStreamCaptureModeThreadLocal));
     const int64_t before = t_launches;
+    const ChainOff off;
     try {
       body();
     } catch (...) {

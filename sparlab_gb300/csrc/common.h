@@ -50,6 +50,35 @@ extern thread_local int64_t t_launches;
     SIMP_CUDA(cudaGetLastError());      \
   } while (0)
 
+// Launch of a kernel whose first statement is chain_start() (kernels.cuh): it
+// may be scheduled while the stream's previous kernel drains, and waits there,
+// before its first access, until that kernel has completed.  The CG iteration,
+// the Lanczos runs and the coarse sweep are chains of kernels of a few
+// microseconds each, where the time from one kernel's end to the next one's
+// start is a third of the total.  ChainOff turns the overlap off for the
+// launches of its scope on the calling thread (bodies of conditional graph
+// nodes).
+extern thread_local int t_chain_off;
+struct ChainOff {
+  ChainOff() { ++t_chain_off; }
+  ~ChainOff() { --t_chain_off; }
+};
+
+template <class... K, class... A>
+void chain_launch(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = t_chain_off ? 0 : 1;
+  SIMP_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+}
+
 // Owning device array (move-only).
 template <class T>
 struct DBuf {

@@ -23,6 +23,7 @@
 #pragma once
 
 #include "common.h"
+#include "kernels.cuh"
 
 #include <algorithm>
 
@@ -102,6 +103,7 @@ template <bool SIGNED>
 __global__ void __launch_bounds__(256) k_sweep_first(const double* __restrict__ m, int n, int kb,
                                                      double* __restrict__ pout, double* __restrict__ piv,
                                                      int* __restrict__ status) {
+  if (!chain_start()) return;
   __shared__ double s[kNB][kNB + 1];
   for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
     const int r = e / kNB, c = e % kNB;
@@ -116,6 +118,7 @@ __global__ void __launch_bounds__(256) k_sweep_first(const double* __restrict__ 
 __global__ void __launch_bounds__(32 * kSweepRows) k_sweep_panel(const double* __restrict__ m, int n, int k0, int kb,
                                                                  const double* __restrict__ p,
                                                                  double* __restrict__ u, double* __restrict__ v) {
+  if (!chain_start()) return;
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * kSweepRows + (threadIdx.x >> 5);
   if (i >= n || (i >= k0 && i < k0 + kb)) return;
@@ -145,6 +148,7 @@ __global__ void __launch_bounds__(256) k_sweep_update(double* __restrict__ m, in
                                                       const double* __restrict__ v,
                                                       const double* __restrict__ p, double* __restrict__ pnext,
                                                       double* __restrict__ piv, int* __restrict__ status) {
+  if (!chain_start()) return;
   const int kt = k0 / kNB;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   __shared__ double vs[kNB][kNB + 1];
@@ -242,13 +246,13 @@ void dense_sweep(double* m, int n, double* panel, double* piv, int* status, cuda
   double* v = u + static_cast<size_t>(n) * kNB;
   double* p[2] = {v + static_cast<size_t>(n) * kNB, v + static_cast<size_t>(n) * kNB + kNB * kNB};
   const int nt = (n + kNB - 1) / kNB;
-  k_sweep_first<SIGNED><<<1, 256, 0, stream>>>(m, n, std::min(kNB, n), p[0], piv, status);
+  chain_launch(k_sweep_first<SIGNED>, 1, 256, 0, stream, m, n, std::min(kNB, n), p[0], piv, status);
   SIMP_CHECK_LAUNCH();
   for (int k0 = 0; k0 < n; k0 += kNB) {
     const int kb = std::min(kNB, n - k0), b = (k0 / kNB) & 1;
-    k_sweep_panel<<<(n + kSweepRows - 1) / kSweepRows, 32 * kSweepRows, 0, stream>>>(m, n, k0, kb, p[b], u, v);
+    chain_launch(k_sweep_panel, (n + kSweepRows - 1) / kSweepRows, 32 * kSweepRows, 0, stream, m, n, k0, kb, p[b], u, v);
     SIMP_CHECK_LAUNCH();
-    k_sweep_update<SIGNED><<<dim3(nt, 2 * nt + 1), 256, 0, stream>>>(m, n, k0, kb, u, v, p[b], p[b ^ 1], piv, status);
+    chain_launch(k_sweep_update<SIGNED>, dim3(nt, 2 * nt + 1), 256, 0, stream, m, n, k0, kb, u, v, p[b], p[b ^ 1], piv, status);
     SIMP_CHECK_LAUNCH();
   }
 }
@@ -257,6 +261,7 @@ void dense_sweep(double* m, int n, double* panel, double* piv, int* status, cuda
 // (I, J), J <= I, per block, written to (I, J) and (J, I).
 __global__ void __launch_bounds__(256) k_sweep_finish(const double* __restrict__ m, double* __restrict__ f,
                                                       int n) {
+  if (!chain_start()) return;
   const int ti = blockIdx.y, tj = blockIdx.x;
   if (tj > ti) return;
   const int r0 = ti * kNB, c0 = tj * kNB;
@@ -281,6 +286,7 @@ __global__ void __launch_bounds__(256) k_sweep_finish(const double* __restrict__
 template <class TX, class TY>
 __global__ void __launch_bounds__(256) k_gemv(const double* __restrict__ m, int n, const TX* __restrict__ x,
                                               TY* __restrict__ y) {
+  if (!chain_start()) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n) return;

@@ -127,6 +127,24 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;
 }
 
+// First statement of every kernel that chain_launch launches, as
+// `if (!chain_start()) return;` (always true: the branch keeps the compiler
+// from moving loads that it takes for invariant above the wait).  All threads
+// wait here until the previous kernel of the stream has completed and its
+// writes are visible; then the next kernel may be scheduled, which waits in
+// turn, so completion stays in stream order.  A grid of more than two blocks an
+// SM lets the next one in only as its blocks end: earlier, the next grid's
+// blocks would fill the slots that happen to be free and the SMs would have
+// unequal shares of it (46800 rows, FP64, 731 blocks after 731: a CG iteration
+// of 227 us against 181 without any overlap).
+constexpr unsigned kChainBlocks = 304;
+__device__ __forceinline__ bool chain_start() {
+  unsigned lane;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%laneid;" : "=r"(lane)::"memory");
+  if (gridDim.x * gridDim.y * gridDim.z <= kChainBlocks) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  return lane < 32u;
+}
+
 // Sum over the grid of one double per block (valid in thread 0): every block
 // stores its partial and takes a ticket, and the last one adds the partials in
 // order, so the value does not depend on which block that is.  True in that
@@ -239,6 +257,7 @@ __global__ void k_convert(const A* __restrict__ a, B* __restrict__ b, i64 n) {
 // three unknowns a node: node order (3 I + k) to component planes (k nodes + I) and back
 template <class A, class B>
 __global__ void k_to_planes(const A* __restrict__ a, B* __restrict__ b, i64 nodes) {
+  if (!chain_start()) return;
   for (i64 I = blockIdx.x * (i64)blockDim.x + threadIdx.x; I < nodes; I += (i64)gridDim.x * blockDim.x)
 #pragma unroll
     for (int k = 0; k < 3; ++k) b[k * nodes + I] = static_cast<B>(a[3 * I + k]);
@@ -246,6 +265,7 @@ __global__ void k_to_planes(const A* __restrict__ a, B* __restrict__ b, i64 node
 
 template <class A, class B>
 __global__ void k_from_planes(const A* __restrict__ a, B* __restrict__ b, i64 nodes) {
+  if (!chain_start()) return;
   for (i64 I = blockIdx.x * (i64)blockDim.x + threadIdx.x; I < nodes; I += (i64)gridDim.x * blockDim.x)
 #pragma unroll
     for (int k = 0; k < 3; ++k) b[3 * I + k] = static_cast<B>(a[k * nodes + I]);
@@ -290,6 +310,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot(const double* __restrict__ 
 __global__ void __launch_bounds__(kRedThreads) k_pcg_begin(const double* __restrict__ r, i32 n, float* __restrict__ b32,
                                                            i32 planes, double* __restrict__ part, PcgScalars* sc,
                                                            PcgPost* host, unsigned seq) {
+  if (!chain_start()) return;
   double s = 0.0;
   for (i32 i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) {
     const double ri = r[i];
@@ -311,6 +332,7 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_begin(const double* __restr
 template <class TZ>
 __global__ void __launch_bounds__(kRedThreads) k_pcg_rz(const double* __restrict__ r, const TZ* __restrict__ z, i32 n,
                                                         i32 planes, double* __restrict__ part, PcgScalars* sc) {
+  if (!chain_start()) return;
   double s = 0.0;
   for (i32 i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads)
     s += r[i] * static_cast<double>(z[planes > 0 ? plane_of(i, planes) : i]);
@@ -329,6 +351,7 @@ template <class TZ>
 __global__ void __launch_bounds__(256) k_pcg_direction(double* __restrict__ p, const TZ* __restrict__ z, i32 n,
                                                        i32 planes, const PcgScalars* __restrict__ sc,
                                                        float2* __restrict__ ps, float* __restrict__ p32) {
+  if (!chain_start()) return;
   const double beta = sc->beta;
   for (i32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double v = static_cast<double>(z[planes > 0 ? plane_of(i, planes) : i]);
@@ -346,6 +369,7 @@ __global__ void __launch_bounds__(256) k_pcg_direction(double* __restrict__ p, c
 // p^T q and alpha
 __global__ void __launch_bounds__(kRedThreads) k_pcg_pq(const double* __restrict__ p, const double* __restrict__ q,
                                                         i32 n, double* __restrict__ part, PcgScalars* sc) {
+  if (!chain_start()) return;
   double s = 0.0;
   for (i32 i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) s += p[i] * q[i];
   double total;
@@ -367,6 +391,7 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_update(double* __restrict__
                                                             const double* __restrict__ q, i32 n,
                                                             float* __restrict__ b32, i32 planes,
                                                             double* __restrict__ part, PcgScalars* sc, PcgPost* host) {
+  if (!chain_start()) return;
   const double alpha = sc->alpha;
   double s = 0.0;
   for (i32 i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) {
@@ -393,6 +418,7 @@ __global__ void __launch_bounds__(kRedThreads) k_pcg_update(double* __restrict__
 template <class TX>
 __global__ void k_cheb_zero(i64 n, const TX* __restrict__ b, const TX* __restrict__ dinv,
                             TX* __restrict__ d, TX* __restrict__ x, const TX* __restrict__ inv_theta) {
+  if (!chain_start()) return;
   const TX it = *inv_theta;
   for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
     const TX di = dinv[i] * b[i] * it;
@@ -457,6 +483,7 @@ __global__ void __launch_bounds__(kRedThreads) k_lz_post(const T* __restrict__ y
                                                          T* __restrict__ w, T* __restrict__ v, i64 n,
                                                          double* __restrict__ alpha, double* __restrict__ part,
                                                          LzScalars* __restrict__ sc) {
+  if (!chain_start()) return;
   if (sc->stop) return;
   const T inv = static_cast<T>(sc->inv), beta = static_cast<T>(sc->last);
   T c = T(0);
@@ -473,6 +500,7 @@ __global__ void __launch_bounds__(kRedThreads) k_lz_norm(const T* __restrict__ s
                                                          const T* __restrict__ v, T* __restrict__ t, i64 n,
                                                          double* __restrict__ ab, double* __restrict__ part,
                                                          LzScalars* __restrict__ sc) {
+  if (!chain_start()) return;
   if (sc->stop) return;
   const T a = static_cast<T>(ab[0]);
   T c = T(0);

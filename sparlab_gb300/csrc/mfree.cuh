@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(128) k_mf2(MfView m, const float* __restrict__
                                              const float* b, float* r, float* __restrict__ dn, float* xs,
                                              const float* __restrict__ dinv, const float* __restrict__ coef, int add_d,
                                              const __grid_constant__ KeQ4 ke) {
+  if (!chain_start()) return;
   const i32 across = (m.nnx + 31) / 32;  // blocks of a row of blocks
   const i32 ix = blockIdx.x % across * 32 + (threadIdx.x & 31), iy = blockIdx.x / across * 4 + (threadIdx.x >> 5);
   if (ix >= m.nnx || iy >= m.nny) return;
@@ -299,6 +300,7 @@ struct MfHalo<true, NZ, TY, TX> {
 
 template <int MODE, int TX = kTX, int TY = kTY, int TZ = kTZ, bool V4 = false>
 __global__ void __launch_bounds__(TX* TY* TZ) k_mf3_tile(MfView m, MfArgs a, const __grid_constant__ KeF32 ke) {
+  if (!chain_start()) return;
   constexpr int NZ = TZ * kNZ;  // node layers of the tile
   __shared__ MfHalo<V4, NZ, TY, TX> xh;
   __shared__ float sc[NZ + 1][TY + 1][TX + 1];
@@ -412,6 +414,7 @@ __global__ void __launch_bounds__(kTX* kTY* kTZ) k_mf3_tile64(MfView m, const do
                                                               const double* __restrict__ x, double* __restrict__ y,
                                                               const double* __restrict__ b,
                                                               const __grid_constant__ KeF64 ke) {
+  if (!chain_start()) return;
   constexpr int NZ = kTZ * kNZ;
   __shared__ double xh[3][NZ + 2][kTY + 2][kTX + 2];
   __shared__ double sc[NZ + 1][kTY + 1][kTX + 1];
@@ -496,6 +499,7 @@ __global__ void __launch_bounds__(256) k_phat_prolong(i32 n, const i32* __restri
                                                       const i32* __restrict__ phat_ptr,
                                                       const float* __restrict__ phat, const float* __restrict__ xc,
                                                       float* __restrict__ t) {
+  if (!chain_start()) return;
   const i32 i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const i32 g = agg[i / 3];
@@ -518,6 +522,7 @@ __global__ void __launch_bounds__(256) k_phat_restrict(i32 naggs, i64 nodes, con
                                                        const i32* __restrict__ phat_ptr,
                                                        const float* __restrict__ phat, const float* __restrict__ t,
                                                        float* __restrict__ bc) {
+  if (!chain_start()) return;
   const i32 g = static_cast<i32>((blockIdx.x * static_cast<i64>(blockDim.x) + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (g >= naggs) return;

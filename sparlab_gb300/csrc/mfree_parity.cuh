@@ -245,6 +245,7 @@ struct ParIo<ParDf> {
 template <int MODE, class AR, int TY>
 __global__ void __launch_bounds__(32 * (TY + 2), 2) k_mf3_par(MfView m, typename ParIo<AR>::Args a,
                                                             const __grid_constant__ typename AR::Ke ke, int chunk) {
+  if (!chain_start()) return;
   using V = typename AR::V;
   using X2 = typename AR::X2;
   using Io = ParIo<AR>;

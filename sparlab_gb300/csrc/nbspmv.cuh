@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(256) k_rows_apply(const i32* __restrict__ node
                                                     const i32* __restrict__ rowptr, const i32* __restrict__ col,
                                                     const TV* __restrict__ val, const TX* __restrict__ x,
                                                     TX* __restrict__ y, const TX* __restrict__ b, i32 rows) {
+  if (!chain_start()) return;
   const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
   const i32 row = static_cast<i32>(t / VS);
   const int lane = static_cast<int>(t % VS);
@@ -108,6 +109,7 @@ __global__ void __launch_bounds__(256) k_rows_cheb_step(i32 rows, const i32* __r
                                                         T* __restrict__ dn, T* __restrict__ x,
                                                         const T* __restrict__ dinv, const T* __restrict__ c12,
                                                         int add_d) {
+  if (!chain_start()) return;
   const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
   const i32 row = static_cast<i32>(t / VS);
   const int lane = static_cast<int>(t % VS);
@@ -132,6 +134,7 @@ __global__ void __launch_bounds__(256) k_rows_cheb_first(i32 rows, const i32* __
                                                          const T* __restrict__ b, T* __restrict__ r,
                                                          T* __restrict__ d, const T* __restrict__ dinv,
                                                          const T* __restrict__ inv_theta) {
+  if (!chain_start()) return;
   const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
   const i32 row = static_cast<i32>(t / VS);
   const int lane = static_cast<int>(t % VS);
@@ -152,6 +155,7 @@ __global__ void __launch_bounds__(256) k_lz_rows(i32 rows, const i32* __restrict
                                                  const T* __restrict__ s, T* __restrict__ w, T* __restrict__ v,
                                                  double* __restrict__ alpha, double* __restrict__ part,
                                                  LzScalars* __restrict__ sc) {
+  if (!chain_start()) return;
   if (sc->stop) return;
   const i64 q = blockIdx.x * (i64)blockDim.x + threadIdx.x;
   const i32 row = static_cast<i32>(q / VS);
@@ -178,6 +182,7 @@ __global__ void __launch_bounds__(256) k_rows_apply_df(const i32* __restrict__ n
                                                        const float2* __restrict__ v, const float2* __restrict__ x,
                                                        double* __restrict__ y,
                                                        const double* __restrict__ b, i32 rows) {
+  if (!chain_start()) return;
   const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
   const i32 row = static_cast<i32>(t / VS);
   const int lane = static_cast<int>(t % VS);
