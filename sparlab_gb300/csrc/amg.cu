@@ -1151,13 +1151,15 @@ void GpuAmg::build_transfer(size_t l) {
   levels.push_back(std::move(nx));
 }
 
-// Launches a warp-per-row-node product with its shared-memory shape; false
-// (nothing launched) when one warp's accumulator would not fit.
+// Launches a row-node product with its shared-memory shape, `per` units (warps
+// or parts of them) a warp and `parts` units a node; false (nothing launched)
+// when one unit's accumulator would not fit.
 template <class T, class... KArgs, class... Args>
-bool launch_rows(const char* name, void (*kernel)(i32, WarpRows, KArgs...), i32 nodes, const WarpRows& w,
+bool launch_rows(const char* name, void (*kernel)(i32, WarpRows, KArgs...), i32 nodes, WarpRows w, int per, int parts,
                  cudaStream_t s, Args... args) {
+  w.acc /= parts;
   const size_t per_warp =
-      static_cast<size_t>(w.acc) * sizeof(T) + static_cast<size_t>(2 * w.slots + kMetaInts + w.inner) * 4;
+      per * (static_cast<size_t>(w.acc) * sizeof(T) + static_cast<size_t>(2 * w.slots + kMetaInts + w.inner) * 4);
   if (per_warp > 200 * 1024) return false;
   // variants: at most 8, 4 or 2 warps (row nodes) per block within a 96 KB
   // (variant 0: the untuned launch) or 192 KB shared-memory budget; a row
@@ -1169,7 +1171,9 @@ bool launch_rows(const char* name, void (*kernel)(i32, WarpRows, KArgs...), i32 
         std::min<size_t>(static_cast<size_t>(kMaxWarps[v]), std::max<size_t>(1, budget / per_warp)));
     const size_t smem = per_warp * warps;
     if (smem > 48 * 1024) raise_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    const i64 blocks = std::max<i64>(1, std::min<i64>((static_cast<i64>(nodes) + warps - 1) / warps, 152 * 64));
+    const i64 units = static_cast<i64>(warps) * per;
+    const i64 blocks =
+        std::max<i64>(1, std::min<i64>((static_cast<i64>(nodes) * parts + units - 1) / units, 152 * 64));
     kernel<<<static_cast<unsigned>(blocks), warps * 32, smem, s>>>(nodes, w, args...);
     SIMP_CHECK_LAUNCH();
   };
@@ -1208,7 +1212,7 @@ static void galerkin_t(GpuAmg& g, Level& lv, Level& nv, bool last, cudaStream_t 
     gather(k_prolongator_gather<T, kExact, 6, 6>);
   } else if (!kExact && bf == 3 && b1 == 3) {
     gather(k_prolongator_gather<T, kExact, 3, 3>);
-  } else if (!launch_rows<T>("prolongator_rows", k_prolongator_rows<T, kExact>, lv.nnodes, lv.wr_p, stream,
+  } else if (!launch_rows<T>("prolongator_rows", k_prolongator_rows<T, kExact>, lv.nnodes, lv.wr_p, 1, 1, stream,
                              lv.d_first.p, nv.d_first.p,
                              lv.d_agg.p, lv.d_apat.view(), lv.a.ptr.p, A(lv.a), lv.d_ppat.view(), lv.p.ptr.p,
                              A(lv.p), lv.phat_ptr.p, phat, lv.dinv64.p, omega)) {
@@ -1225,26 +1229,45 @@ static void galerkin_t(GpuAmg& g, Level& lv, Level& nv, bool last, cudaStream_t 
         lv.d_ppat.view(), lv.p.ptr.p, A(lv.p));
     SIMP_CHECK_LAUNCH();
   }
-  auto ap_rows = [&](auto kernel) {
-    return launch_rows<T>("ap_rows", kernel, lv.nnodes, lv.wr_ap, stream, lv.d_first.p, lv.d_apat.view(), lv.a.ptr.p,
-                          A(lv.a),
-                          lv.d_ppat.view(), lv.p.ptr.p, A(lv.p), lv.d_appat.view(), lv.ap.ptr.p, A(lv.ap));
+  auto ap_rows = [&](auto kernel, int per, int parts) {
+    return launch_rows<T>("ap_rows", kernel, lv.nnodes, lv.wr_ap, per, parts, stream, lv.d_first.p, lv.d_apat.view(),
+                          lv.a.ptr.p, A(lv.a), lv.d_ppat.view(), lv.p.ptr.p, A(lv.p), lv.d_appat.view(), lv.ap.ptr.p,
+                          A(lv.ap));
   };
-  auto rap_rows = [&](auto kernel) {
-    return launch_rows<T>("rap_rows", kernel, nv.nnodes, lv.wr_rap, stream, nv.d_first.p, lv.d_first.p,
+  auto rap_rows = [&](auto kernel, int parts) {
+    return launch_rows<T>("rap_rows", kernel, nv.nnodes, lv.wr_rap, 1, parts, stream, nv.d_first.p, lv.d_first.p,
                           lv.d_rpat.view(),
                           lv.r.ptr.p, A(lv.r), lv.d_appat.view(), lv.ap.ptr.p, A(lv.ap), nv.d_apat.view(),
                           nv.a.ptr.p, raw);
   };
   // compile-time node widths for the common shapes: 3-D level 0 (3 -> 6),
-  // coarse 3-D (6 -> 6), 2-D level 0 (2 -> 3), coarse 2-D (3 -> 3)
+  // coarse 3-D (6 -> 6), 2-D level 0 (2 -> 3), coarse 2-D (3 -> 3).  The exact
+  // FP64 products are bound by the FP64 pipe, which takes a whole warp's time
+  // whatever the active lanes: half warps where a P row is short (62 x 38 x 30
+  // nodes, 3 -> 6: 2.51 -> 2.23 ms), and parts of a node's rows where the nodes
+  // give an SM fewer than 16 units (AP) or 64 (RAP, whose units differ more in
+  // length; 140 nodes, 6 -> 6: 1.09 -> 0.63 ms).  The FP32 ones are bound by
+  // instruction issue and by latency, and lose by either (193 x 97 x 97 nodes,
+  // 3 -> 6 by half warps: 6.86 -> 7.41 ms; 127 nodes, 6 -> 6 by rows: 0.51 ->
+  // 0.92 ms).
   constexpr bool X = std::is_same<T, double>::value;
+  constexpr int H = X ? 16 : 32, PER = 32 / H;
   const int b0 = uniform_block(lv.first);
-  const bool ap_done = (b0 == 3 && b1 == 6)   ? ap_rows(k_ap_rows<T, X, 3, 6>)
-                       : (b0 == 6 && b1 == 6) ? ap_rows(k_ap_rows<T, X, 6, 6>)
-                       : (b0 == 2 && b1 == 3) ? ap_rows(k_ap_rows<T, X, 2, 3>)
-                       : (b0 == 3 && b1 == 3) ? ap_rows(k_ap_rows<T, X, 3, 3>)
-                                              : ap_rows(k_ap_rows<T, X, 0, 0>);
+  bool ap_done = false;
+  if constexpr (X) {
+    if (lv.nnodes < 16 * 152)
+      ap_done = (b0 == 3 && b1 == 6)   ? ap_rows(k_ap_rows<T, X, 3, 6, H, 1>, PER, 3)
+                : (b0 == 6 && b1 == 6) ? ap_rows(k_ap_rows<T, X, 6, 6, 32, 1>, 1, 6)
+                : (b0 == 2 && b1 == 3) ? ap_rows(k_ap_rows<T, X, 2, 3, H, 1>, PER, 2)
+                : (b0 == 3 && b1 == 3) ? ap_rows(k_ap_rows<T, X, 3, 3, H, 1>, PER, 3)
+                                       : false;
+  }
+  if (!ap_done)
+    ap_done = (b0 == 3 && b1 == 6)   ? ap_rows(k_ap_rows<T, X, 3, 6, H, 3>, PER, 1)
+              : (b0 == 6 && b1 == 6) ? ap_rows(k_ap_rows<T, X, 6, 6, 32, 6>, 1, 1)
+              : (b0 == 2 && b1 == 3) ? ap_rows(k_ap_rows<T, X, 2, 3, H, 2>, PER, 1)
+              : (b0 == 3 && b1 == 3) ? ap_rows(k_ap_rows<T, X, 3, 3, H, 3>, PER, 1)
+                                     : ap_rows(k_ap_rows<T, X, 0, 0, 32, 0>, 1, 1);
   if (!ap_done) {
     const i64 th = static_cast<i64>(lv.n) * 32;
     k_product_ap<32, T><<<grid_for(th, 256), 256, 0, stream>>>(
@@ -1252,11 +1275,25 @@ static void galerkin_t(GpuAmg& g, Level& lv, Level& nv, bool last, cudaStream_t 
         lv.d_ppat.view(), lv.p.ptr.p, A(lv.p), lv.d_appat.view(), lv.ap.ptr.p, A(lv.ap));
     SIMP_CHECK_LAUNCH();
   }
-  const bool rap_done = (b1 == 6 && b0 == 3)   ? rap_rows(k_rap_rows<T, X, 6, 3>)
-                        : (b1 == 6 && b0 == 6) ? rap_rows(k_rap_rows<T, X, 6, 6>)
-                        : (b1 == 3 && b0 == 2) ? rap_rows(k_rap_rows<T, X, 3, 2>)
-                        : (b1 == 3 && b0 == 3) ? rap_rows(k_rap_rows<T, X, 3, 3>)
-                                               : rap_rows(k_rap_rows<T, X, 0, 0>);
+  bool rap_done = false;
+  if constexpr (X) {
+    if (nv.nnodes < 4 * 152)
+      rap_done = (b1 == 6 && b0 == 3)   ? rap_rows(k_rap_rows<T, X, 6, 3, 1>, 6)
+                 : (b1 == 6 && b0 == 6) ? rap_rows(k_rap_rows<T, X, 6, 6, 1>, 6)
+                                        : false;
+    if (!rap_done && nv.nnodes < 64 * 152)
+      rap_done = (b1 == 6 && b0 == 3)   ? rap_rows(k_rap_rows<T, X, 6, 3, 2>, 3)
+                 : (b1 == 6 && b0 == 6) ? rap_rows(k_rap_rows<T, X, 6, 6, 2>, 3)
+                 : (b1 == 3 && b0 == 2) ? rap_rows(k_rap_rows<T, X, 3, 2, 1>, 3)
+                 : (b1 == 3 && b0 == 3) ? rap_rows(k_rap_rows<T, X, 3, 3, 1>, 3)
+                                        : false;
+  }
+  if (!rap_done)
+    rap_done = (b1 == 6 && b0 == 3)   ? rap_rows(k_rap_rows<T, X, 6, 3, 6>, 1)
+               : (b1 == 6 && b0 == 6) ? rap_rows(k_rap_rows<T, X, 6, 6, 6>, 1)
+               : (b1 == 3 && b0 == 2) ? rap_rows(k_rap_rows<T, X, 3, 2, 3>, 1)
+               : (b1 == 3 && b0 == 3) ? rap_rows(k_rap_rows<T, X, 3, 3, 3>, 1)
+                                      : rap_rows(k_rap_rows<T, X, 0, 0, 0>, 1);
   if (!rap_done) {
     const i64 th = static_cast<i64>(nv.n) * 32;
     k_product_rap<32, T><<<grid_for(th, 256), 256, 0, stream>>>(
@@ -1267,7 +1304,7 @@ static void galerkin_t(GpuAmg& g, Level& lv, Level& nv, bool last, cudaStream_t 
   // FP64 copy of the coarse operator where the FP64 path or the coarse
   // factorisation needs it
   double* out64 = (!f32 || last) ? nv.a.v64.p : nullptr;
-  k_symmetrize<T, T><<<grid_for(nv.n, 128), 128, 0, stream>>>(nv.n, nv.d_node_of.p, nv.d_first.p, nv.d_apat.view(),
+  k_symmetrize<T, T><<<grid_for(static_cast<i64>(nv.n) * 32, 256), 256, 0, stream>>>(nv.n, nv.d_node_of.p, nv.d_first.p, nv.d_apat.view(),
                                                               nv.a.ptr.p, lv.d_sym_t.p, raw, A(nv.a), f32 ? out64 : nullptr);
   SIMP_CHECK_LAUNCH();
 }
@@ -1306,7 +1343,7 @@ void GpuAmg::coarse_factorize() {
   piv_.alloc(n);
   panel_.alloc(sweep_panel_size(n));
   SIMP_CUDA(cudaMemsetAsync(swept_.p, 0, nn * sizeof(double), stream));
-  k_dense_from_csr<<<grid_for(n, 128), 128, 0, stream>>>(n, lv.a.ptr.p, lv.a.col.p, lv.a.v64.p, swept_.p);
+  k_dense_from_csr<<<grid_for(static_cast<i64>(n) * 32, 256), 256, 0, stream>>>(n, lv.a.ptr.p, lv.a.col.p, lv.a.v64.p, swept_.p);
   SIMP_CHECK_LAUNCH();
   SIMP_CUDA(cudaMemsetAsync(dstatus.p, 0, sizeof(int), stream));
   dense_sweep<false>(swept_.p, n, panel_.p, piv_.p, dstatus.p, stream);

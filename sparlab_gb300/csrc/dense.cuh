@@ -297,10 +297,11 @@ __global__ void __launch_bounds__(256) k_gemv(const double* __restrict__ m, int 
   if (lane == 0) y[warp] = static_cast<TY>(s);
 }
 
+// one warp a row
 __global__ void k_dense_from_csr(int n, const i32* __restrict__ ptr, const i32* __restrict__ col,
                                  const double* __restrict__ val, double* __restrict__ a) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
-    for (i32 k = ptr[r]; k < ptr[r + 1]; ++k) a[(size_t)r * n + col[k]] = val[k];
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5)
+    for (i32 k = ptr[r] + (threadIdx.x & 31); k < ptr[r + 1]; k += 32) a[(size_t)r * n + col[k]] = val[k];
 }
 
 // a = K - s G densely, K and G on the same CSR pattern (a zeroed before).

@@ -9,8 +9,16 @@
 // product and one rounded add per term.  Within one left slot the warp's
 // lanes own distinct outputs; __syncwarp orders consecutive slots.
 //
-// Shared memory per warp: the accumulator (rows x row length of T), the
+// Shared memory per unit: the accumulator (rows x row length of T), the
 // output slots and their offsets, and the positions of the inner row's slots.
+//
+// A unit is a warp or half of one (G lanes), and takes all rows of a node or
+// RW of them.  Half warps where a left slot's inner row is short (P rows of a
+// few aggregates: 15 to 25 columns, which leave 32 lanes half empty), both
+// halves in lockstep: every loop runs to the longer half's count and every
+// barrier is the whole warp's.  Parts of a node's rows where the nodes are too
+// few to fill the chip.  Each row's terms keep their order, so all splits give
+// the same bits; amg.cu has the rule and what it measured.
 #pragma once
 
 #include "amg.h"
@@ -39,10 +47,10 @@ struct WarpSmem {
 constexpr int kMetaInts = 8 * kChunk + 1;
 
 template <class T>
-__device__ __forceinline__ T* warp_setup(const WarpRows& w, int warps, int warp, unsigned char* smem, WarpSmem& m) {
-  T* acc = reinterpret_cast<T*>(smem) + static_cast<size_t>(warp) * w.acc;
-  int* base = reinterpret_cast<int*>(reinterpret_cast<T*>(smem) + static_cast<size_t>(warps) * w.acc) +
-              static_cast<size_t>(warp) * (2 * w.slots + kMetaInts + w.inner);
+__device__ __forceinline__ T* warp_setup(const WarpRows& w, int units, int unit, unsigned char* smem, WarpSmem& m) {
+  T* acc = reinterpret_cast<T*>(smem) + static_cast<size_t>(unit) * w.acc;
+  int* base = reinterpret_cast<int*>(reinterpret_cast<T*>(smem) + static_cast<size_t>(units) * w.acc) +
+              static_cast<size_t>(unit) * (2 * w.slots + kMetaInts + w.inner);
   m.sl = base;
   m.soff = m.sl + w.slots;
   m.mj = m.soff + w.slots;
@@ -67,23 +75,32 @@ __device__ __forceinline__ int lower_slot(const int* sl, int ns, i32 h) {
   return lo;
 }
 
-// Stage the output slots of a row node and zero its accumulator rows.
-template <class T>
-__device__ __forceinline__ void warp_begin(NodeView out, i32 node, int nrows, int len, int lane, const WarpSmem& m,
-                                           T* acc) {
-  const i32 s0 = out.ptr[node], ns = out.ptr[node + 1] - s0;
-  for (int q = lane; q < ns; q += 32) {
-    m.sl[q] = out.nbr[s0 + q];
-    m.soff[q] = out.off[s0 + q];
+// Stage the ns output slots of a row node and zero its accumulator rows.
+template <int G, class T>
+__device__ __forceinline__ void warp_begin(NodeView out, i32 node, int ns, int nrows, int len, int lane,
+                                           const WarpSmem& m, T* acc) {
+  if (ns > 0) {
+    const i32 s0 = out.ptr[node];
+    for (int q = lane; q < ns; q += G) {
+      m.sl[q] = out.nbr[s0 + q];
+      m.soff[q] = out.off[s0 + q];
+    }
+    for (int q = lane; q < nrows * len; q += G) acc[q] = T(0);
   }
-  for (int q = lane; q < nrows * len; q += 32) acc[q] = T(0);
   __syncwarp();
 }
 
-// Phase 1 + 2 for one chunk of the left operand's slots [t0, t0 + nt):
+// the largest x of the warp's units
+template <int G>
+__device__ __forceinline__ int unit_max(int x) {
+  return G == 32 ? x : __reduce_max_sync(0xffffffffu, x);
+}
+
+// Phase 1 + 2 for one chunk of the left operand's slots [t0, t0 + nt), nt <= G:
 // metadata of each slot's inner row node (lanes over slots), then the
 // accumulator position of every (slot, inner slot) pair (lanes over pairs).
 // left: the left operand's node pattern; inner: the inner rows' pattern.
+template <int G>
 __device__ __forceinline__ void warp_chunk(NodeView left, i32 t0, int nt, const i32* __restrict__ first,
                                            NodeView inner, const i32* __restrict__ irow, int ns, int lane,
                                            const WarpSmem& m) {
@@ -102,15 +119,15 @@ __device__ __forceinline__ void warp_chunk(NodeView left, i32 t0, int nt, const 
   }
   int incl = nu;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+  for (int o = 1; o < G; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o, G);
     if (lane >= o) incl += v;
   }
   if (lane < nt) m.mpre[lane] = incl - nu;
-  const int npairs = __shfl_sync(0xffffffffu, incl, 31);
+  const int npairs = __shfl_sync(0xffffffffu, incl, G - 1, G);
   if (lane == 0) m.mpre[nt] = npairs;
   __syncwarp();
-  for (int q = lane; q < npairs; q += 32) {
+  for (int q = lane; q < npairs; q += G) {
     int lo = 0, hi = nt - 1;  // the last slot t with mpre[t] <= q
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -153,11 +170,12 @@ __device__ __forceinline__ constexpr int wmax() { return W > 0 ? W : 6; }
 template <int W>
 __device__ __forceinline__ bool within(int k, int n) { return W > 0 ? true : k < n; }
 
-// AP = A P: warp per fine node I; inner rows are P's rows of I's neighbours J.
+// AP = A P: unit per fine node I (and part of its rows); inner rows are P's
+// rows of I's neighbours J.
 // acc(ka, pos(c)) += sum_kb A((I,ka),(J,kb)) P((J,kb), c), kb ascending.
 // NR: unknowns per node of this level (rows of I and of every J), B1: of the
-// next level (0 = not uniform).
-template <class T, bool EXACT, int NR, int B1>
+// next level (0 = not uniform); RW: rows of a unit (NR, or a divisor).
+template <class T, bool EXACT, int NR, int B1, int G, int RW>
 __global__ void __launch_bounds__(256) k_ap_rows(i32 nodes, WarpRows w, const i32* __restrict__ first,
                                                  NodeView a, const i32* __restrict__ arow,
                                                  const T* __restrict__ aval, NodeView p,
@@ -165,63 +183,70 @@ __global__ void __launch_bounds__(256) k_ap_rows(i32 nodes, WarpRows w, const i3
                                                  NodeView ap, const i32* __restrict__ aprow,
                                                  T* __restrict__ apval) {
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr int MR = wmax<NR>();
-  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int MR = wmax<NR>(), MW = wmax<RW>(), NG = 32 / G, PARTS = RW > 0 ? NR / RW : 1;
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & (G - 1);
+  const int unit = warp * NG + (threadIdx.x & 31) / G;
   WarpSmem m;
-  T* acc = warp_setup<T>(w, warps, warp, smem, m);
-  for (i32 I = blockIdx.x * warps + warp; I < nodes; I += gridDim.x * warps) {
-    const i32 r0 = first[I], nr = NR > 0 ? NR : first[I + 1] - r0;
-    const int ns = ap.ptr[I + 1] - ap.ptr[I];
-    if (nr == 0 || ns == 0) continue;
-    const i32 L = aprow[r0 + 1] - aprow[r0];
-    const i32 abase = arow[r0], LA = arow[r0 + 1] - arow[r0];
-    warp_begin<T>(ap, I, nr, L, lane, m, acc);
-    for (i32 t0 = a.ptr[I]; t0 < a.ptr[I + 1]; t0 += kChunk) {
-      const int nt = min(kChunk, a.ptr[I + 1] - t0);
-      warp_chunk(a, t0, nt, first, p, prow, ns, lane, m);
-      for (int t = 0; t < nt; ++t) {
-        const int sJ = NR > 0 ? NR : m.msj[t], Lp = m.mlen[t];
-        if (NR == 0 && sJ == 0) continue;
-        T ar[MR][MR];
-        const T* av = aval + abase + m.maux[t];
+  T* acc = warp_setup<T>(w, warps * NG, unit, smem, m);
+  const i32 items = nodes * PARTS;
+  for (i32 i0 = (blockIdx.x * warps + warp) * NG; i0 < items; i0 += gridDim.x * warps * NG) {
+    const i32 item = i0 + unit % NG, I = min(item / PARTS, nodes - 1);
+    const int ka0 = (item % PARTS) * (RW > 0 ? RW : 0);
+    const i32 r0 = first[I], nr = RW > 0 ? RW : first[I + 1] - r0;
+    const int ns = item < items && nr > 0 ? ap.ptr[I + 1] - ap.ptr[I] : 0;
+    if (unit_max<G>(ns) == 0) continue;
+    const i32 L = ns > 0 ? aprow[r0 + 1] - aprow[r0] : 0;
+    const i32 abase = ns > 0 ? arow[r0] : 0, LA = ns > 0 ? arow[r0 + 1] - abase : 0;
+    const i32 ts = a.ptr[I], left = ns > 0 ? a.ptr[I + 1] - ts : 0;
+    warp_begin<G, T>(ap, I, ns, nr, L, lane, m, acc);
+    for (i32 t0 = 0; t0 < unit_max<G>(left); t0 += G) {
+      const int nt = max(0, min(G, left - t0));
+      warp_chunk<G>(a, ts + t0, nt, first, p, prow, ns, lane, m);
+      for (int t = 0; t < unit_max<G>(nt); ++t) {
+        const int sJ = NR > 0 ? NR : t < nt ? m.msj[t] : 0, Lp = t < nt ? m.mlen[t] : 0;
+        if (Lp > 0) {
+          T ar[MW][MR];
+          const T* av = aval + abase + m.maux[t] + ka0 * LA;
 #pragma unroll
-        for (int ka = 0; ka < MR; ++ka)
+          for (int ka = 0; ka < MW; ++ka)
 #pragma unroll
-          for (int kb = 0; kb < MR; ++kb)
-            ar[ka][kb] = (within<NR>(ka, nr) && within<NR>(kb, sJ)) ? av[ka * LA + kb] : T(0);
-        const T* pv = pval + m.mrow[t];
-        for (int c = lane; c < Lp; c += 32) {
-          T pc[MR];
+            for (int kb = 0; kb < MR; ++kb)
+              ar[ka][kb] = (within<RW>(ka, nr) && within<NR>(kb, sJ)) ? av[ka * LA + kb] : T(0);
+          const T* pv = pval + m.mrow[t];
+          for (int c = lane; c < Lp; c += G) {
+            T pc[MR];
 #pragma unroll
-          for (int kb = 0; kb < MR; ++kb) pc[kb] = within<NR>(kb, sJ) ? pv[kb * Lp + c] : T(0);
-          const int pos = pair_pos<B1>(c, t, m, p.off);
+            for (int kb = 0; kb < MR; ++kb) pc[kb] = within<NR>(kb, sJ) ? pv[kb * Lp + c] : T(0);
+            const int pos = pair_pos<B1>(c, t, m, p.off);
 #pragma unroll
-          for (int ka = 0; ka < MR; ++ka) {
-            if (within<NR>(ka, nr)) {
-              T v = acc[ka * L + pos];
+            for (int ka = 0; ka < MW; ++ka) {
+              if (within<RW>(ka, nr)) {
+                T v = acc[ka * L + pos];
 #pragma unroll
-              for (int kb = 0; kb < MR; ++kb)
-                if (within<NR>(kb, sJ)) v = term<EXACT>(v, ar[ka][kb], pc[kb]);
-              acc[ka * L + pos] = v;
+                for (int kb = 0; kb < MR; ++kb)
+                  if (within<NR>(kb, sJ)) v = term<EXACT>(v, ar[ka][kb], pc[kb]);
+                acc[ka * L + pos] = v;
+              }
             }
           }
         }
         __syncwarp();
       }
     }
-    for (int ka = 0; ka < nr; ++ka) {
-      T* out = apval + aprow[r0 + ka];
-      for (int q = lane; q < L; q += 32) out[q] = acc[ka * L + q];
+    for (int ka = 0; ns > 0 && ka < nr; ++ka) {
+      T* out = apval + aprow[r0 + ka0 + ka];
+      for (int q = lane; q < L; q += G) out[q] = acc[ka * L + q];
     }
     __syncwarp();
   }
 }
 
-// RAW = R (AP): warp per coarse node g; inner rows are AP's rows of the fine
-// nodes I of R's row g.  acc(kg, pos(c)) += sum_ka R((g,kg),(I,ka)) AP((I,ka), c).
+// RAW = R (AP): warp per coarse node g (and part of its rows); inner rows are
+// AP's rows of the fine nodes I of R's row g.
+// acc(kg, pos(c)) += sum_ka R((g,kg),(I,ka)) AP((I,ka), c).
 // NC: unknowns per coarse node (rows of g, and the AP column-node width),
-// NF: per fine node (0 = not uniform).
-template <class T, bool EXACT, int NC, int NF>
+// NF: per fine node (0 = not uniform); RW: rows of a warp (NC, or a divisor).
+template <class T, bool EXACT, int NC, int NF, int RW>
 __global__ void __launch_bounds__(256) k_rap_rows(i32 nodes, WarpRows w, const i32* __restrict__ first1,
                                                   const i32* __restrict__ first, NodeView r,
                                                   const i32* __restrict__ rrow, const T* __restrict__ rval,
@@ -229,30 +254,32 @@ __global__ void __launch_bounds__(256) k_rap_rows(i32 nodes, WarpRows w, const i
                                                   const T* __restrict__ apval, NodeView c,
                                                   const i32* __restrict__ crow, T* __restrict__ cval) {
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr int MC = wmax<NC>(), MF = wmax<NF>();
+  constexpr int MW = wmax<RW>(), MF = wmax<NF>(), PARTS = RW > 0 ? NC / RW : 1;
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   WarpSmem m;
   T* acc = warp_setup<T>(w, warps, warp, smem, m);
-  for (i32 g = blockIdx.x * warps + warp; g < nodes; g += gridDim.x * warps) {
-    const i32 r0 = first1[g], nr = NC > 0 ? NC : first1[g + 1] - r0;
+  for (i32 item = blockIdx.x * warps + warp; item < nodes * PARTS; item += gridDim.x * warps) {
+    const i32 g = item / PARTS;
+    const int kg0 = (item % PARTS) * (RW > 0 ? RW : 0);
+    const i32 r0 = first1[g], nr = RW > 0 ? RW : first1[g + 1] - r0;
     const int ns = c.ptr[g + 1] - c.ptr[g];
     if (nr == 0 || ns == 0) continue;
     const i32 L = crow[r0 + 1] - crow[r0];
     const i32 rbase = rrow[r0], LR = rrow[r0 + 1] - rrow[r0];
-    warp_begin<T>(c, g, nr, L, lane, m, acc);
+    warp_begin<32, T>(c, g, ns, nr, L, lane, m, acc);
     for (i32 t0 = r.ptr[g]; t0 < r.ptr[g + 1]; t0 += kChunk) {
       const int nt = min(kChunk, r.ptr[g + 1] - t0);
-      warp_chunk(r, t0, nt, first, ap, aprow, ns, lane, m);
+      warp_chunk<32>(r, t0, nt, first, ap, aprow, ns, lane, m);
       for (int t = 0; t < nt; ++t) {
         const int sI = NF > 0 ? NF : m.msj[t], La = m.mlen[t];
         if (NF == 0 && sI == 0) continue;
-        T rr[MC][MF];
-        const T* rv = rval + rbase + m.maux[t];
+        T rr[MW][MF];
+        const T* rv = rval + rbase + m.maux[t] + kg0 * LR;
 #pragma unroll
-        for (int kg = 0; kg < MC; ++kg)
+        for (int kg = 0; kg < MW; ++kg)
 #pragma unroll
           for (int ka = 0; ka < MF; ++ka)
-            rr[kg][ka] = (within<NC>(kg, nr) && within<NF>(ka, sI)) ? rv[kg * LR + ka] : T(0);
+            rr[kg][ka] = (within<RW>(kg, nr) && within<NF>(ka, sI)) ? rv[kg * LR + ka] : T(0);
         const T* pv = apval + m.mrow[t];
         for (int cc = lane; cc < La; cc += 32) {
           T pc[MF];
@@ -260,8 +287,8 @@ __global__ void __launch_bounds__(256) k_rap_rows(i32 nodes, WarpRows w, const i
           for (int ka = 0; ka < MF; ++ka) pc[ka] = within<NF>(ka, sI) ? pv[ka * La + cc] : T(0);
           const int pos = pair_pos<NC>(cc, t, m, ap.off);
 #pragma unroll
-          for (int kg = 0; kg < MC; ++kg) {
-            if (within<NC>(kg, nr)) {
+          for (int kg = 0; kg < MW; ++kg) {
+            if (within<RW>(kg, nr)) {
               T v = acc[kg * L + pos];
 #pragma unroll
               for (int ka = 0; ka < MF; ++ka)
@@ -274,7 +301,7 @@ __global__ void __launch_bounds__(256) k_rap_rows(i32 nodes, WarpRows w, const i
       }
     }
     for (int kg = 0; kg < nr; ++kg) {
-      T* out = cval + crow[r0 + kg];
+      T* out = cval + crow[r0 + kg0 + kg];
       for (int q = lane; q < L; q += 32) out[q] = acc[kg * L + q];
     }
     __syncwarp();
@@ -300,7 +327,7 @@ __global__ void __launch_bounds__(256) k_prolongator_rows(
     if (nr == 0 || ns == 0) continue;
     const i32 L = prow[r0 + 1] - prow[r0];
     const i32 abase = arow[r0], LA = arow[r0 + 1] - arow[r0];
-    warp_begin<T>(p, I, nr, L, lane, m, acc);
+    warp_begin<32, T>(p, I, ns, nr, L, lane, m, acc);
     for (i32 t0 = a.ptr[I]; t0 < a.ptr[I + 1]; t0 += kChunk) {
       const int nt = min(kChunk, a.ptr[I + 1] - t0);
       // per neighbour: its unknowns, its aggregate's position and rank

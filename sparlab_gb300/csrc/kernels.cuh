@@ -740,15 +740,19 @@ __global__ void __launch_bounds__(256) k_product_rap(
   }
 }
 
-// A_c = (RAW + RAW^T) / 2 on the (structurally symmetric) coarse pattern.
+// A_c = (RAW + RAW^T) / 2 on the (structurally symmetric) coarse pattern: a
+// warp a row, a lane a slot (a thread a row was a serial walk of strided reads:
+// 0.95 -> 0.34 ms for 26136 nodes of six unknowns, 94 -> 10 us for 127).
 template <class T, class TO>
 __global__ void k_symmetrize(i32 nc, const i32* __restrict__ node_of1, const i32* __restrict__ first1,
                              NodeView c, const i32* __restrict__ crow, const i32* __restrict__ tslot,
                              const T* __restrict__ raw, TO* __restrict__ out, double* __restrict__ out64) {
-  for (i64 row = blockIdx.x * (i64)blockDim.x + threadIdx.x; row < nc; row += (i64)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (i64 row = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5; row < nc;
+       row += ((i64)gridDim.x * blockDim.x) >> 5) {
     const i32 g = node_of1[row];
     const i32 lc = static_cast<i32>(row) - first1[g];
-    for (i32 s = c.ptr[g]; s < c.ptr[g + 1]; ++s) {
+    for (i32 s = c.ptr[g] + lane; s < c.ptr[g + 1]; s += 32) {
       const i32 h = c.nbr[s];
       const i32 st = tslot[s];
       const i32 base = crow[row] + c.off[s];
