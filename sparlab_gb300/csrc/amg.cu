@@ -66,6 +66,13 @@ namespace {
 // for the arithmetic type.
 template <class TA, class F>
 void with_shape(const NbOp& op, F&& f) {
+  if constexpr (std::is_same<TA, float>::value) {
+    // the coarse levels' 3-D operators and long restrictions: a warp a node
+    if (op.six) {
+      f(std::integral_constant<int, kNodeWarp>{}, std::integral_constant<int, 6>{});
+      return;
+    }
+  }
   auto lanes = [&](auto b) {
     switch (std::is_same<TA, double>::value ? op.lanes64 : op.lanes32) {
       case 32: f(std::integral_constant<int, 32>{}, b); break;
@@ -106,7 +113,8 @@ int red_blocks(i64 n) { return grid_for(n, kRedThreads, kRedBlocks); }
 
 // One thread per (row, lane); no grid-stride loop in the row kernels.
 unsigned rows_grid(const NbOp& op, int vs) {
-  const i64 blocks = (static_cast<i64>(op.rows) * vs + 255) / 256;
+  const i64 threads = vs == kNodeWarp ? static_cast<i64>(op.nodes) * 32 : static_cast<i64>(op.rows) * vs;
+  const i64 blocks = (threads + 255) / 256;
   return static_cast<unsigned>(std::max<i64>(blocks, 1));
 }
 
@@ -165,6 +173,12 @@ int row_lanes(const DevCsr& c) {
   // flight per warp, which the per-row index chain (row -> node -> slots ->
   // x) needs to hide its latency (P_0 at 192x96x96: 93 against 150 us)
   return avg >= 256 ? 32 : (avg >= 64 ? 8 : 4);
+}
+
+// Operators whose FP32 products take a warp a node (node_rows_dot).  Rows of
+// fewer than 64 values leave half of its lanes idle; those keep 4 lanes a row.
+bool six_by_six(const NbOp& op, const std::vector<i32>& row_first) {
+  return op.block == 6 && op.lanes32 >= 8 && uniform_block(row_first) == 6;
 }
 
 // Per-precision views of a level's arrays.
@@ -610,6 +624,7 @@ void GpuAmg::make_ops(size_t l) {
   lv.opA.rows = lv.n;
   lv.opA.lanes32 = row_lanes<float>(lv.a);
   lv.opA.lanes64 = row_lanes<double>(lv.a);
+  lv.opA.six = six_by_six(lv.opA, lv.first);
   if (l + 1 < levels.size()) {
     Level& nv = *levels[l + 1];
     lv.opP.nodes = lv.nnodes;
@@ -622,6 +637,7 @@ void GpuAmg::make_ops(size_t l) {
     lv.opP.rows = lv.n;
     lv.opP.lanes32 = row_lanes<float>(lv.p);
     lv.opP.lanes64 = row_lanes<double>(lv.p);
+    lv.opP.six = six_by_six(lv.opP, lv.first);
     lv.opR.nodes = nv.nnodes;
     lv.opR.row_first = nv.d_first.p;
     lv.opR.pat = lv.d_rpat.view();
@@ -632,6 +648,7 @@ void GpuAmg::make_ops(size_t l) {
     lv.opR.rows = nv.n;
     lv.opR.lanes32 = row_lanes<float>(lv.r);
     lv.opR.lanes64 = row_lanes<double>(lv.r);
+    lv.opR.six = six_by_six(lv.opR, nv.first);
   }
 }
 

@@ -56,6 +56,81 @@ __device__ __forceinline__ TA lane_dot(i32 len, int lane, i32 s0, const i32* __r
   return s;
 }
 
+// Where a row's result ends up: the row, its sum, and whether this lane has it.
+template <class T>
+struct RowResult {
+  i32 row;
+  T s;
+  bool holds;
+};
+
+// The six rows of a 3-D coarse node by one warp (FP32; VS = kNodeWarp): a lane
+// takes two columns of the node at a time, reads x and the slot record once
+// and the six rows' values as 8-byte pairs (row lengths are multiples of six,
+// so pairs are aligned and stay within a block): 8 loads for 12 products where
+// the row kernel's lanes issue 36, which bound it (0.55 of HBM on level 1 of
+// 192x96x96: its design pass 68.7 -> 64.7 ms, 96x48x48's 17.9 -> 16.9).  The lanes then halve the set of rows that they hold at each
+// step; lanes 4k .. 4k + 3 end with row k.
+constexpr int kNodeWarp = 64;
+__device__ __forceinline__ RowResult<float> node_rows_dot(i32 rows, NodeView pat, const i32* __restrict__ rowptr,
+                                                          const float* __restrict__ val,
+                                                          const float* __restrict__ x) {
+  const i32 node = static_cast<i32>((blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  const bool valid = 6 * node < rows;
+  float s[8] = {};
+  if (valid) {
+    const i32 k0 = rowptr[6 * node], len = rowptr[6 * node + 1] - k0, s0 = pat.ptr[node];
+    const float* v = val + k0;
+#pragma unroll 2
+    for (i32 w = 2 * lane; w < len; w += 64) {
+      const i32 t = w / 6;
+      const float2 xv = *reinterpret_cast<const float2*>(x + 6 * pat.nbr[s0 + t] + (w - 6 * t));
+      float2 a[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) a[k] = *reinterpret_cast<const float2*>(v + k * len + w);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) s[k] = fmaf(a[k].y, xv.y, fmaf(a[k].x, xv.x, s[k]));
+    }
+  }
+#pragma unroll
+  for (int step = 0; step < 3; ++step) {
+    const int half = 4 >> step, off = 16 >> step;
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i >= half) continue;
+      const float give = up ? s[i] : s[i + half], keep = up ? s[i + half] : s[i];
+      s[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+    }
+  }
+  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 2);
+  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+  return {6 * node + (lane >> 2), s[0], valid && (lane & 3) == 0 && lane < 24};
+}
+
+template <int VS, int B, class TV, class TX, class TA>
+__device__ __forceinline__ RowResult<TA> row_result(i32 rows, const i32* __restrict__ node_of, NodeView pat,
+                                                    const i32* __restrict__ rowptr, const i32* __restrict__ col,
+                                                    const TV* __restrict__ val, const TX* __restrict__ x) {
+  if constexpr (VS == kNodeWarp) {
+    return node_rows_dot(rows, pat, rowptr, val, x);
+  } else {
+    const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
+    const i32 row = static_cast<i32>(t / VS);
+    const int lane = static_cast<int>(t % VS);
+    TA s = TA(0);
+    if (row < rows) {
+      const i32 k0 = rowptr[row], len = rowptr[row + 1] - k0;
+      const i32 s0 = B > 0 ? pat.ptr[node_of[row]] : 0;
+      s = lane_dot<VS, B, TV, TX, TA>(len, lane, s0, pat.nbr, col + k0, val + k0, x);
+    }
+#pragma unroll
+    for (int o = VS / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, VS);
+    return {row, s, row < rows && lane == 0};
+  }
+}
+
 // mode 0: y = A x ; 1: y = b - A x ; 2: y += A x.  TA is the arithmetic
 // type (FP64 rows get VS = 4: GB300's FP64 rate is 1/64 of FP32, and a short
 // reduction keeps the FP64 pipe on the products).
@@ -65,37 +140,12 @@ __global__ void __launch_bounds__(256) k_rows_apply(const i32* __restrict__ node
                                                     const TV* __restrict__ val, const TX* __restrict__ x,
                                                     TX* __restrict__ y, const TX* __restrict__ b, i32 rows) {
   if (!chain_start()) return;
-  const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  const i32 row = static_cast<i32>(t / VS);
-  const int lane = static_cast<int>(t % VS);
-  TA s = TA(0);
-  if (row < rows) {
-    const i32 k0 = rowptr[row], len = rowptr[row + 1] - k0;
-    const i32 s0 = B > 0 ? pat.ptr[node_of[row]] : 0;
-    s = lane_dot<VS, B, TV, TX, TA>(len, lane, s0, pat.nbr, col + k0, val + k0, x);
-  }
-#pragma unroll
-  for (int o = VS / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, VS);
-  if (row < rows && lane == 0) {
+  const auto [row, s, holds] = row_result<VS, B, TV, TX, TA>(rows, node_of, pat, rowptr, col, val, x);
+  if (holds) {
     if (MODE == 0) y[row] = static_cast<TX>(s);
     else if (MODE == 1) y[row] = b[row] - static_cast<TX>(s);
     else y[row] += static_cast<TX>(s);
   }
-}
-
-template <int VS, int B, class TV, class TX>
-__device__ __forceinline__ TX rows_dot(i32 row, int lane, bool valid, const i32* __restrict__ node_of, NodeView pat,
-                                       const i32* __restrict__ rowptr, const i32* __restrict__ col,
-                                       const TV* __restrict__ val, const TX* __restrict__ x) {
-  TX s = TX(0);
-  if (valid) {
-    const i32 k0 = rowptr[row], len = rowptr[row + 1] - k0;
-    const i32 s0 = B > 0 ? pat.ptr[node_of[row]] : 0;
-    s = lane_dot<VS, B, TV, TX, TX>(len, lane, s0, pat.nbr, col + k0, val + k0, x);
-  }
-#pragma unroll
-  for (int o = VS / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, VS);
-  return s;
 }
 
 // Chebyshev step: r = r_in - A d ; dn = c1 d + c2 dinv r ; x = (x [+ d]) + dn,
@@ -110,12 +160,8 @@ __global__ void __launch_bounds__(256) k_rows_cheb_step(i32 rows, const i32* __r
                                                         const T* __restrict__ dinv, const T* __restrict__ c12,
                                                         int add_d) {
   if (!chain_start()) return;
-  const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  const i32 row = static_cast<i32>(t / VS);
-  const int lane = static_cast<int>(t % VS);
-  const bool valid = row < rows;
-  const T s = rows_dot<VS, B, T, T>(row, lane, valid, node_of, pat, rowptr, col, val, d);
-  if (valid && lane == 0) {
+  const auto [row, s, holds] = row_result<VS, B, T, T, T>(rows, node_of, pat, rowptr, col, val, d);
+  if (holds) {
     const T ri = r_in[row] - s;
     r[row] = ri;
     const T di = c12[0] * d[row] + c12[1] * dinv[row] * ri;
@@ -135,12 +181,8 @@ __global__ void __launch_bounds__(256) k_rows_cheb_first(i32 rows, const i32* __
                                                          T* __restrict__ d, const T* __restrict__ dinv,
                                                          const T* __restrict__ inv_theta) {
   if (!chain_start()) return;
-  const i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  const i32 row = static_cast<i32>(t / VS);
-  const int lane = static_cast<int>(t % VS);
-  const bool valid = row < rows;
-  const T s = rows_dot<VS, B, T, T>(row, lane, valid, node_of, pat, rowptr, col, val, x);
-  if (valid && lane == 0) {
+  const auto [row, s, holds] = row_result<VS, B, T, T, T>(rows, node_of, pat, rowptr, col, val, x);
+  if (holds) {
     const T ri = b[row] - s;
     r[row] = ri;
     d[row] = dinv[row] * ri * *inv_theta;
@@ -157,15 +199,11 @@ __global__ void __launch_bounds__(256) k_lz_rows(i32 rows, const i32* __restrict
                                                  LzScalars* __restrict__ sc) {
   if (!chain_start()) return;
   if (sc->stop) return;
-  const i64 q = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  const i32 row = static_cast<i32>(q / VS);
-  const int lane = static_cast<int>(q % VS);
-  const bool valid = row < rows;
-  const T y = rows_dot<VS, B, T, T>(row, lane, valid, node_of, pat, rowptr, col, val, t);
+  const auto [row, y, holds] = row_result<VS, B, T, T, T>(rows, node_of, pat, rowptr, col, val, t);
   T c = T(0);
-  if (valid && lane == 0) c = lz_row(y, row, s, w, v, static_cast<T>(sc->inv), static_cast<T>(sc->last));
+  if (holds) c = lz_row(y, row, s, w, v, static_cast<T>(sc->inv), static_cast<T>(sc->last));
   double total;
-  if (grid_sum(rows_block_sum<VS>(c), part, &sc->ticket, total)) *alpha = total;
+  if (grid_sum(rows_block_sum<VS == kNodeWarp ? 4 : VS>(c), part, &sc->ticket, total)) *alpha = total;
 }
 
 // Double-float operator (mixed precision's CG operator): values stored as
