@@ -1657,8 +1657,10 @@ void GpuAmg::pcg_tail(SolveWork& w, float2* psplit) {
     using TZ = std::remove_cv_t<std::remove_pointer_t<decltype(z)>>;
     chain_launch(k_pcg_rz<TZ>, red_blocks(n), kRedThreads, 0, stream, residual(w), z, n, planes, w.part.p, w.scalars());
     SIMP_CHECK_LAUNCH();
-    chain_launch(k_pcg_direction<TZ>, grid_for(n, 256), 256, 0, stream, w.pp.p, z, n, planes, w.scalars(), psplit,
-                                                           mf_cg() ? w.p32.p : nullptr);
+    // four values a thread where that still gives every SM eight blocks
+    const bool four = n >= 4 * 256 * 8 * 152;
+    chain_launch(four ? k_pcg_direction<TZ, 4> : k_pcg_direction<TZ, 1>, (static_cast<i64>(n) + (four ? 1023 : 255)) / (four ? 1024 : 256),
+                 256, 0, stream, w.pp.p, z, n, planes, w.scalars(), psplit, mf_cg() ? w.p32.p : nullptr);
     SIMP_CHECK_LAUNCH();
   };
   if (mixed()) {
