@@ -683,12 +683,20 @@ def run_own(args):
     nnz = prob.nnz
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / (kms * 1e-3) / 1e9
+    if args.precision == "fp64":
+        operator = f"k_rows_apply<4,{spec.dim},0,double> (level-0 K_ff operator of the CG, FP64 values; FP64-pipe bound on GB300)"
+    elif alg_bytes < 8.0 * nnz:  # no stored values among its bytes
+        operator = ("k_mf3_par<0,ParDf> (level-0 operator of the CG, matrix-free in the parity basis, double-float "
+                    "arithmetic on the FP32 pipes; bound by their issue rate)")
+    else:
+        operator = (f"k_rows_apply_df<4,{spec.dim},0> (level-0 K_ff operator of the CG, double-float values and "
+                    "arithmetic on the FP32 pipes)")
     traffic = None
     prof = os.path.join(ROOT, "profiles", "spmv_traffic.json")
     if os.path.exists(prof):
         with open(prof) as f:
             d = json.load(f)
-        if d.get("workload") == spec.name:
+        if d.get("workload") == spec.name and d.get("kernel", "").startswith(operator.split(" ")[0]):
             traffic = d.get("traffic_bytes_per_launch")
 
     def timed_run(precision, with_surrogate):
@@ -783,10 +791,7 @@ def run_own(args):
                 "oracle_check": oracle_check},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic,
-                     "kernel": (f"k_rows_apply<4,{spec.dim},0,double> (level-0 K_ff operator of the CG, "
-                                "FP64 values; FP64-pipe bound on GB300)" if args.precision == "fp64" else
-                                f"k_rows_apply_df<4,{spec.dim},0> (level-0 K_ff operator of the CG, "
-                                "double-float values and arithmetic on the FP32 pipes)"),
+                     "kernel": operator,
                      "bytes_per_launch": alg_bytes, "ms_per_launch": kms,
                      "peak_kind": f"{peak_kind} hbm_gbs (burst copy)"},
         "cpu_baseline": cpu,
