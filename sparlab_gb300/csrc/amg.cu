@@ -176,9 +176,11 @@ int row_lanes(const DevCsr& c) {
 }
 
 // Operators whose FP32 products take a warp a node (node_rows_dot).  Rows of
-// fewer than 64 values leave half of its lanes idle; those keep 4 lanes a row.
+// fewer than 64 values leave half of its lanes idle (4 lanes a row), and few
+// nodes with rows of 256 and more, the restrictions, too many SMs (32 lanes a
+// row: 17.4 us per restriction at 192x96x96 against 23.4).
 bool six_by_six(const NbOp& op, const std::vector<i32>& row_first) {
-  return op.block == 6 && op.lanes32 >= 8 && uniform_block(row_first) == 6;
+  return op.block == 6 && op.lanes32 == 8 && uniform_block(row_first) == 6;
 }
 
 // Per-precision views of a level's arrays.

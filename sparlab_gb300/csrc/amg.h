@@ -71,7 +71,7 @@ struct NbOp {
   const i32* node_of = nullptr; // row -> row node
   i32 rows = 0;
   int lanes32 = 8, lanes64 = 4; // lanes per row of the FP32 / FP64 kernels
-  bool six = false;             // six rows a node, six columns a block, rows of 64 values and more
+  bool six = false;             // six rows a node, six columns a block, rows of 64 to 255 values
   // lanes per row of the double-float kernels (level 0): 4 -- each lane's
   // longer row chain and twice the rows per warp hide the gathers' latency
   // better than 8 lanes (0.700 against 0.779 ms per launch at 192x96x96)
