@@ -59,9 +59,23 @@ void check_encode(CUresult r, const char* what) {
 
 }  // namespace
 
+// What both convolution kernels ask of their arguments, checked on the host
+// before any device call.  The inputs come in by TMA, the weights by TMA
+// (k_conv_tc) or 16-byte cp.async (k_conv_march): all must start on 16 bytes.
+void check_conv(const ConvSpec& s) {
+  auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  for (int k = 0; k < s.nseg; ++k) {
+    if (s.cseg[k] != 16 && s.cseg[k] != 32 && s.cseg[k] != 64)
+      throw Error(kBadInput, "surrogate: input segments must have 16, 32 or 64 channels");
+    if (!aligned(s.in[k])) throw Error(kBadInput, "surrogate: activations must be 16-byte aligned");
+  }
+  if (s.n % 16 || s.n < 16 || s.n > 128) throw Error(kBadInput, "surrogate: output columns must be 16..128, step 16");
+  if (s.nout > 1 && s.out_c[0] % 16) throw Error(kBadInput, "surrogate: split outputs at a multiple of 16 columns");
+  if (!s.w || !aligned(s.w)) throw Error(kBadInput, "surrogate: weights must be 16-byte aligned");
+}
+
 // Channels-last BF16 activations [nz][ny][nx][c]: boxes of (c, 32, rows, 1).
 CUtensorMap act_map(const void* base, int c, int nx, int ny, int nz, int rows) {
-  if (reinterpret_cast<uintptr_t>(base) % 16) throw Error(kBadInput, "surrogate: activations must be 16-byte aligned");
   CUtensorMap m;
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(c), static_cast<cuuint64_t>(nx), static_cast<cuuint64_t>(ny),
                               static_cast<cuuint64_t>(nz)};
@@ -78,7 +92,6 @@ CUtensorMap act_map(const void* base, int c, int nx, int ny, int nz, int rows) {
 
 // Weights [27 n rows][k] (K contiguous): boxes of (c, n) at column offset k0.
 CUtensorMap weight_map(const void* base, int k, int n, int c) {
-  if (reinterpret_cast<uintptr_t>(base) % 16) throw Error(kBadInput, "surrogate: weights must be 16-byte aligned");
   CUtensorMap m;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(27) * n};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k) * 2};
@@ -137,21 +150,18 @@ void conv_launch(const ConvSpec& s, cudaStream_t stream) {
   p.relu = s.relu;
   p.nout = s.nout;
   p.status = s.status;
+  check_conv(s);
   int ktot = 0;
   for (int k = 0; k < s.nseg; ++k) {
-    if (s.cseg[k] != 16 && s.cseg[k] != 32 && s.cseg[k] != 64)
-      throw Error(kBadInput, "surrogate: input segments must have 16, 32 or 64 channels");
     p.cseg[k] = s.cseg[k];
     ktot += s.cseg[k];
   }
-  if (s.n % 16 || s.n < 16 || s.n > 128) throw Error(kBadInput, "surrogate: output columns must be 16..128, step 16");
   for (int k = 0; k < s.nout; ++k) {
     p.out_c[k] = s.out_c[k];
     p.out_pitch[k] = s.out_pitch[k];
     p.out_f32[k] = s.out_f32[k];
     p.out[k] = s.out[k];
   }
-  if (s.nout > 1 && s.out_c[0] % 16) throw Error(kBadInput, "surrogate: split outputs at a multiple of 16 columns");
   if (conv_march_launch(s, p, ktot, stream)) return;
   const CUtensorMap a0 = act_map(s.in[0], s.cseg[0], s.nx, s.ny, s.nz, conv::kTileY);
   const CUtensorMap a1 = s.nseg > 1 ? act_map(s.in[1], s.cseg[1], s.nx, s.ny, s.nz, conv::kTileY) : a0;
@@ -401,6 +411,7 @@ int simp_conv3d_bf16(int32_t nx, int32_t ny, int32_t nz, int32_t nseg, const voi
       s.out_pitch[k] = out_pitch[k];
       s.out_f32[k] = out_f32[k];
     }
+    sg::check_conv(s);
     DBuf<int> st(1);
     st.zero();
     s.status = st.p;

@@ -47,6 +47,7 @@ struct WgradSpec {
   int* status = nullptr;  // device word set on a wait that ran out
 };
 
+void check_conv(const ConvSpec& s);
 CUtensorMap act_map(const void* base, int c, int nx, int ny, int nz, int rows);
 CUtensorMap weight_map(const void* base, int k, int n, int c);
 void conv_launch(const ConvSpec& s, cudaStream_t stream);
