@@ -875,8 +875,7 @@ struct LzBufs<float> {
 // Inverse diagonal and the m Lanczos steps of a level (Multigrid.cpp:288-327,
 // 718-747).  T = double: FP64 vectors and operator.  T = float (the FP32 reuse
 // setups): FP32 vectors and the FP32 operator the smoother uses (matrix-free
-// on a structured level 0), with the scalars and the sums across warps in
-// FP64.
+// on a structured level 0), with the scalars and the sums of rows in FP64.
 template <class T>
 void GpuAmg::lanczos(size_t l, int m, double* ab) {
   Level& lv = *levels[l];
@@ -895,13 +894,13 @@ void GpuAmg::lanczos(size_t l, int m, double* ab) {
   const int vs = f32 ? lv.opA.lanes32 : lv.opA.lanes64;
   lz_part_.alloc(std::max<size_t>(lz_part_.n, std::max<size_t>(kRedBlocks, rows_grid(lv.opA, vs))));
   double* pt = lz_part_.p;
-  k_lz_reset<<<1, 1, 0, stream>>>(sc, lv.lz_norm);
+  k_lz_reset<<<1, 1, 0, stream>>>(sc);
   SIMP_CHECK_LAUNCH();
   // (level 0's dinv32 after a first setup follows when its order is known)
   if (mixed()) lv.dinv32.alloc(n);
   k_level_start<T><<<grid_for(n, 256), 256, 0, stream>>>(n, lv.d_node_of.p, lv.d_first.p, lv.d_self.p,
                                                          lv.d_apat.view(), lv.a.ptr.p, values, lv.lz_start.p,
-                                                         lv.dinv64.p, lv.dinv32.p, s, w, t, v, planes, sc);
+                                                         lv.lz_norm, lv.dinv64.p, lv.dinv32.p, s, w, t, v, planes, sc);
   SIMP_CHECK_LAUNCH();
   if constexpr (f32)
     if (matrix_free) lz_y_.alloc(static_cast<size_t>(n));

@@ -449,14 +449,18 @@ __global__ void k_cheb_zero(i64 n, const TX* __restrict__ b, const TX* __restric
 // product and k_lz_post), then k_lz_norm; the last block of each adds the
 // partials in order.  The vector of a step stays unnormalised: u = beta_{j-1}
 // v_j is in w and t = s u is the operator's input, scaled in the rows'
-// epilogue, so no pass divides by beta.  FP32 vectors (the mixed-precision
-// reuse setups) take FP32 arithmetic with FP64 scalars and sums across warps:
-// GB300 runs FP64 at 1/64 of the FP32 rate.
+// epilogue, so no pass divides by beta (the first one is the start vector over
+// its norm, divided in FP64, with beta_0 = 1).  FP32 vectors (the
+// mixed-precision reuse setups) take FP32 arithmetic with FP64 scalars, and a
+// row's products are added up in FP64: GB300 runs FP64 at 1/64 of the FP32
+// rate, so a block of rows leaves its products in shared memory and one warp
+// adds them, 7 FP64 additions a block where sums in every warp take 32.
 // ---------------------------------------------------------------------------
 // Device scalars of a level's Lanczos run (alpha_j and beta_j follow the host's
 // order in an array of their own).
 struct LzScalars {
-  double inv;       // 1 / beta of the last step (the start vector's norm before the first)
+  double inv;       // 1 / beta of the last step (1 before the first) ...
+  double inv_low;   // ... and what rounding cut off it
   double last;      // that beta
   int stop;         // breakdown: the later steps change nothing
   int bad;          // first non-positive diagonal entry, or kLzGood
@@ -465,28 +469,40 @@ struct LzScalars {
 };
 constexpr int kLzGood = 0x7fffffff;
 
-// Sum over the lanes that hold a row's result (lane 0 of each VS group).
+// Sum in FP64 of the block's row values, which lane 0 of each VS group holds
+// (256 threads; valid in thread 0).
 template <int VS, class T>
 __device__ __forceinline__ double rows_block_sum(T v) {
-  __shared__ double part[8];
-#pragma unroll
-  for (int o = VS; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = static_cast<double>(v);
+  constexpr int kRows = 256 / VS;
+  __shared__ T row_value[kRows];
+  if (threadIdx.x % VS == 0) row_value[threadIdx.x / VS] = v;
   __syncthreads();
   double s = 0.0;
-  if (threadIdx.x == 0)
+  if (threadIdx.x < 32) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) s += part[k];
+    for (int k = threadIdx.x; k < kRows; k += 32) s += static_cast<double>(row_value[k]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  }
   return s;
 }
+
+// x / beta.  FP64 multiplies by 1 / beta in two parts, which rounds once, as the
+// division would; FP32 by the rounded 1 / beta.
+struct LzScale {
+  double inv, low;
+  __device__ __forceinline__ LzScale(const LzScalars& sc) : inv(sc.inv), low(sc.inv_low) {}
+  __device__ __forceinline__ float operator()(float x) const { return x * static_cast<float>(inv); }
+  __device__ __forceinline__ double operator()(double x) const { return fma(x, inv, x * low); }
+};
 
 // u_j and v_{j-1} of row i become w = S A v_j - beta_{j-1} v_{j-1} and v_j, from
 // y = (A t)_i; returns w_i v_i.
 template <class T>
-__device__ __forceinline__ T lz_row(T y, i64 i, const T* __restrict__ s, T* __restrict__ w, T* __restrict__ v, T inv,
-                                    T beta) {
-  const T vn = w[i] * inv;
-  const T wn = y * inv * s[i] - beta * v[i];
+__device__ __forceinline__ T lz_row(T y, i64 i, const T* __restrict__ s, T* __restrict__ w, T* __restrict__ v,
+                                    const LzScale& over_beta, T beta) {
+  const T vn = over_beta(w[i]);
+  const T wn = over_beta(y) * s[i] - beta * v[i];
   w[i] = wn;
   v[i] = vn;
   return wn * vn;
@@ -500,10 +516,11 @@ __global__ void __launch_bounds__(kRedThreads) k_lz_post(const T* __restrict__ y
                                                          LzScalars* __restrict__ sc) {
   if (!chain_start()) return;
   if (sc->stop) return;
-  const T inv = static_cast<T>(sc->inv), beta = static_cast<T>(sc->last);
+  const LzScale over_beta(*sc);
+  const T beta = static_cast<T>(sc->last);
   T c = T(0);
   for (i64 i = blockIdx.x * (i64)kRedThreads + threadIdx.x; i < n; i += (i64)gridDim.x * kRedThreads)
-    c += lz_row(y[i], i, s, w, v, inv, beta);
+    c += lz_row(y[i], i, s, w, v, over_beta, beta);
   double total;
   if (grid_sum(block_sum<kRedThreads>(static_cast<double>(c)), part, &sc->ticket, total)) *alpha = total;
 }
@@ -530,28 +547,31 @@ __global__ void __launch_bounds__(kRedThreads) k_lz_norm(const T* __restrict__ s
     const double b = sqrt(total);
     ab[1] = b;
     if (!(b > 1.0e-12 * fabs(ab[0]))) sc->stop = 1;
+    const double inv = 1.0 / b;
     sc->last = b;
-    sc->inv = 1.0 / b;
+    sc->inv = inv;
+    sc->inv_low = fma(-inv, b, 1.0) * inv;
   }
 }
 
-// The scalars before a level's first kernel: norm = ||start||.
-__global__ void k_lz_reset(LzScalars* sc, double norm) {
-  sc->inv = 1.0 / norm;
-  sc->last = norm;
+// The scalars before a level's first kernel.
+__global__ void k_lz_reset(LzScalars* sc) {
+  sc->inv = 1.0;
+  sc->inv_low = 0.0;
+  sc->last = 1.0;
   sc->stop = 0;
   sc->bad = kLzGood;
   sc->ticket = 0;
 }
 
 // Inverse diagonal of a level (1 / a_ii; the first entry that is not positive
-// is recorded) and the Lanczos start: s = sqrt(1 / a_ii), w = start, t = s w,
-// v = 0.  planes > 0: dinv32, s, w, t and v in component planes of that many
+// is recorded) and the Lanczos start: s = sqrt(1 / a_ii), w = start / norm,
+// t = s w, v = 0.  planes > 0: dinv32, s, w, t and v in component planes of that many
 // nodes (three unknowns a node).
 template <class T>
 __global__ void k_level_start(i32 n, const i32* __restrict__ node_of, const i32* __restrict__ first,
                               const i32* __restrict__ self_slot, NodeView a, const i32* __restrict__ rowptr,
-                              const T* __restrict__ val, const double* __restrict__ start, double* __restrict__ dinv,
+                              const T* __restrict__ val, const double* __restrict__ start, double norm, double* __restrict__ dinv,
                               float* __restrict__ dinv32, T* __restrict__ s, T* __restrict__ w, T* __restrict__ t,
                               T* __restrict__ v, i64 planes, LzScalars* __restrict__ sc) {
   for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
@@ -564,7 +584,7 @@ __global__ void k_level_start(i32 n, const i32* __restrict__ node_of, const i32*
     dinv[i] = inv;
     const i64 o = planes > 0 ? (i % 3) * planes + i / 3 : i;
     if (dinv32) dinv32[o] = static_cast<float>(inv);
-    const T si = static_cast<T>(sqrt(inv)), wi = static_cast<T>(start[i]);
+    const T si = static_cast<T>(sqrt(inv)), wi = static_cast<T>(start[i] / norm);
     s[o] = si;
     w[o] = wi;
     t[o] = si * wi;

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(256) k_lz_rows(i32 rows, const i32* __restrict
   if (sc->stop) return;
   const auto [row, y, holds] = row_result<VS, B, T, T, T>(rows, node_of, pat, rowptr, col, val, t);
   T c = T(0);
-  if (holds) c = lz_row(y, row, s, w, v, static_cast<T>(sc->inv), static_cast<T>(sc->last));
+  if (holds) c = lz_row(y, row, s, w, v, LzScale(*sc), static_cast<T>(sc->last));
   double total;
   if (grid_sum(rows_block_sum<VS == kNodeWarp ? 4 : VS>(c), part, &sc->ticket, total)) *alpha = total;
 }
