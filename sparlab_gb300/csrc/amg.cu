@@ -7,6 +7,7 @@
 #include "dense.cuh"
 #include "galerkin.cuh"
 #include "kernels.cuh"
+#include "march.h"
 #include "mfree.cuh"
 #include "mfree_parity.cuh"
 #include "mfree_tc.cuh"
@@ -272,11 +273,8 @@ void mf3_tc(const MfOp& mf, const MfArgs& a, const KeF32& ke, cudaStream_t s) {
   SIMP_CHECK_LAUNCH();
 }
 
-// Launch of the parity kernel: the chunking of the z march that takes the
-// fewest block steps, waves x (layers + 2) -- a block's march costs its layers
-// and about two more to fill and drain (97x49x49: one wave of 5 layers 12.8
-// us, 4 layers in 1.2 waves 14.9, 8 layers in 0.6 waves 14.9).  Every
-// chunking gives the same values.
+// Launch of the parity kernel, its z march split by march_layers.  Every split
+// gives the same values.
 template <class K>
 dim3 par_grid(const MfOp& mf, int rows, K kernel, int* layers) {
   static std::mutex mu;
@@ -297,16 +295,7 @@ dim3 par_grid(const MfOp& mf, int rows, K kernel, int* layers) {
   }
   const i64 nnz = mf.nz + 1;
   const dim3 xy((mf.nnx + kParCols - 1) / kParCols, (mf.nny + rows - 1) / rows);
-  const i64 columns = static_cast<i64>(xy.x) * xy.y;
-  i64 best = nnz, steps = std::numeric_limits<i64>::max();
-  for (i64 l = 1; l <= nnz; ++l) {
-    const i64 blocks = columns * ((nnz + l - 1) / l);
-    const i64 s = (blocks + slots - 1) / slots * (l + 2);
-    if (s < steps) {
-      steps = s;
-      best = l;
-    }
-  }
+  const i64 best = march_layers(static_cast<i64>(xy.x) * xy.y, nnz, slots);
   *layers = static_cast<int>(best);
   return dim3(xy.x, xy.y, static_cast<unsigned>((nnz + best - 1) / best));
 }
