@@ -979,15 +979,12 @@ void GpuAmg::numeric_level(size_t l) {
     lv.c2.push_back(2.0 * rn / delta);
     rho = rn;
   }
-  // the kernels read them from device memory: [1 / theta, c1_0, c2_0, ...,
-  // 0, 0] (the closing pair is the degree-1 step's)
+  // the kernels read them from device memory: [1 / theta, c1_0, c2_0, ...]
   std::vector<double> coef{lv.inv_theta};
   for (size_t k = 0; k < lv.c1.size(); ++k) {
     coef.push_back(lv.c1[k]);
     coef.push_back(lv.c2[k]);
   }
-  coef.push_back(0.0);
-  coef.push_back(0.0);
   const double omega = opt.damping / lv.lambda;
   lv.cheb64.alloc(coef.size());
   lv.cheb32.alloc(coef.size());
@@ -1575,7 +1572,10 @@ void GpuAmg::smooth(SolveWork& w, size_t l, bool zero_guess) {
     }
     std::swap(d, e);
   }
-  if (opt.degree == 1 && !zero_guess) nb_cheb_step<T>(lv.opA, A, d, r, r, e, x, dinv, V<T>::cheb(lv) + 1, 1, stream);
+  if (opt.degree == 1 && !zero_guess) {  // no step has added d yet
+    chain_launch(k_add_to<T>, grid_for(n, 256), 256, 0, stream, n, d, x);
+    SIMP_CHECK_LAUNCH();
+  }
 }
 
 template <class T>

@@ -442,6 +442,13 @@ __global__ void k_cheb_zero(i64 n, const TX* __restrict__ b, const TX* __restric
   }
 }
 
+// x += d
+template <class TX>
+__global__ void k_add_to(i64 n, const TX* __restrict__ d, TX* __restrict__ x) {
+  if (!chain_start()) return;
+  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) x[i] += d[i];
+}
+
 // ---------------------------------------------------------------------------
 // Lanczos on S A S, S = D^-1/2 (src/fem/Multigrid.cpp:288-327), two launches a
 // step instead of eight: the operator's rows with the step's vector update and
