@@ -835,7 +835,7 @@ int simp_problem_kff(simp_problem* p, const double* scale, int32_t* rowptr, int3
       if (!scale) throw Error(kBadInput, "simp_problem_kff: values need element factors");
       DBuf<double> s;
       s.upload(scale, static_cast<size_t>(g.ne), g.amg.stream);
-      g.assemble(s.p, true);
+      g.assemble(s.p, nullptr, true);
       l0.a.v64.download(val, static_cast<size_t>(l0.a.nnz), g.amg.stream);
       SIMP_CUDA(cudaStreamSynchronize(g.amg.stream));
     }

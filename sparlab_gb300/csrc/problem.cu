@@ -471,14 +471,14 @@ void GpuProblem::assemble_into(const double* elem, const double* scale, bool exa
   SIMP_CHECK_LAUNCH();
 }
 
-void GpuProblem::assemble(const double* scale, bool exact) {
+void GpuProblem::assemble(const double* scale, const float2* scale2, bool exact) {
   Level& l0 = *amg.levels.front();
   if (l0.nnodes == 0) return;
   const GridView g = grid_of(d);
   const unsigned blocks = static_cast<unsigned>((l0.nnodes + kAsmTile - 1) / kAsmTile);
   const size_t smem = assemble_smem(d.dim);
   const int threads = assemble_threads(d.dim);
-  auto launch = [&](auto kernel, const float2* scale2, double* v64, float* hi, float2* pair) {
+  auto launch = [&](auto kernel, double* v64, float* hi, float2* pair) {
     raise_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     kernel<<<blocks, threads, smem, amg.stream>>>(g, l0.nnodes, l0.d_first.p, gnode.p, cmask.p, nmask.p,
                                                   l0.d_apat.view(), l0.a.ptr.p, ke_d.p, scale, scale2, v64, hi,
@@ -486,8 +486,8 @@ void GpuProblem::assemble(const double* scale, bool exact) {
     SIMP_CHECK_LAUNCH();
   };
   if (!amg.mixed()) {
-    if (exact) launch(k_assemble_tiles<true, false>, nullptr, l0.a.v64.p, nullptr, nullptr);
-    else launch(k_assemble_tiles<false, false>, nullptr, l0.a.v64.p, nullptr, nullptr);
+    if (exact) launch(k_assemble_tiles<true, false>, l0.a.v64.p, nullptr, nullptr);
+    else launch(k_assemble_tiles<false, false>, l0.a.v64.p, nullptr, nullptr);
     return;
   }
   // mixed: the double-float split (hi = the FP32 values of the preconditioner,
@@ -496,12 +496,12 @@ void GpuProblem::assemble(const double* scale, bool exact) {
   l0.a.v32.alloc(static_cast<size_t>(l0.a.nnz));
   if (!amg.par_cg()) l0.a.v2.alloc(static_cast<size_t>(l0.a.nnz));
   if (exact) {
-    launch(k_assemble_tiles<true, false>, nullptr, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
+    launch(k_assemble_tiles<true, false>, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
   } else if (!amg.opt.reuse) {
     // every setup rebuilds the hierarchy from FP64 values
-    launch(k_assemble_tiles<false, false>, nullptr, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
+    launch(k_assemble_tiles<false, false>, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
   } else {
-    launch(k_assemble_tiles<false, true>, sf2.p, nullptr, l0.a.v32.p, l0.a.v2.p);
+    launch(k_assemble_tiles<false, true>, nullptr, l0.a.v32.p, l0.a.v2.p);
   }
   amg.level0_fp32_fresh = true;
 }
@@ -563,7 +563,7 @@ void GpuProblem::evaluate_prepare() {
   }
   // the structure-defining first assembly is bit-exact (the aggregates come
   // from its values); later ones use fused multiply-adds
-  assemble(sf.p, !structure_built_);
+  assemble(sf.p, sf2.p, !structure_built_);
   amg.setup(!structure_built_);
   structure_built_ = true;
   last_compliance.assign(static_cast<size_t>(d.nloads), 0.0);
