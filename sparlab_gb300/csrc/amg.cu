@@ -916,10 +916,9 @@ void GpuAmg::lanczos(size_t l, int m, double* ab) {
 }
 
 // inverse diagonal and lambda_max(D^-1 A) of one level (Multigrid.cpp:718-747)
-void GpuAmg::numeric_level(size_t l) {
+void GpuAmg::numeric_level(size_t l, bool fp32) {
   Level& lv = *levels[l];
   const i32 n = lv.n;
-  const bool fp32 = mixed() && ready_ && lv.a.v32.p != nullptr;
   make_ops(l);
   lv.dinv64.alloc(n);
   // Lanczos on D^-1/2 A D^-1/2 with the reference's start vector (its norm
@@ -1383,9 +1382,36 @@ void GpuAmg::coarse_solve(SolveWork& w, size_t l) {
   SIMP_CHECK_LAUNCH();
 }
 
+// FP32 Galerkin products carry about 1e-7 of the entries into the next level.
+// Where the coarse operators are near singular (beams 20 to 40 times as long as
+// they are high: their bending stiffness is what is left of entries 1e5 to 1e7
+// times as large), that can make a pivot of the coarsest one negative although
+// the matrix is positive definite: 90 of 190 cantilevers of 120 to 480 x 4 to 12 x 4
+// to 12 cells failed so at the second setup.  FP64 decides then.
 void GpuAmg::setup(bool structure_changed) {
-  const auto t0 = std::chrono::steady_clock::now();
   const bool reuse = opt.reuse && !structure_changed && ready_;
+  if (!reuse) fp64_reuse_ = false;
+  // Reused structure in mixed mode: FP32 numerics; a new structure is set up
+  // in FP64 so the aggregates come from the FP64 values.
+  const bool fp32 = reuse && fp32_reuse();
+  try {
+    setup_once(reuse, fp32);
+    return;
+  } catch (const Error& e) {
+    if (!fp32 || (e.code != kUnderConstrained && e.code != kBreakdown)) throw;
+  }
+  fp64_reuse_ = true;
+  try {
+    if (write_level0_fp64) write_level0_fp64();
+    setup_once(true, false);
+  } catch (...) {
+    fp64_reuse_ = false;  // the matrix, not FP32
+    throw;
+  }
+}
+
+void GpuAmg::setup_once(bool reuse, bool fp32) {
+  const auto t0 = std::chrono::steady_clock::now();
   if (mf.enabled) {
     mf.status = mf_status.p;
     mf.tensor = mf.dim == 3 && opt.tensor_cores != 0;
@@ -1399,15 +1425,12 @@ void GpuAmg::setup(bool structure_changed) {
     l0.naggs = 0;
     ready_ = false;
   }
-  // Reused structure in mixed mode: FP32 numerics; a new structure is set up
-  // in FP64 so the aggregates come from the FP64 values.
-  const bool fp32 = mixed() && reuse;
   if (mixed() && !level0_fp32_fresh) refresh_level0_fp32();
   level0_fp32_fresh = false;
   const size_t reused_levels = levels.size();
   size_t l = 0;
   while (true) {
-    numeric_level(l);
+    numeric_level(l, fp32);
     Level& lv = *levels[l];
     const bool stop = reuse ? (l + 1 == reused_levels)
                             : (lv.n <= opt.coarse_size || static_cast<int>(l) + 1 >= opt.max_levels);

@@ -16,6 +16,7 @@
 #include "common.h"
 #include "structure.h"
 
+#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -251,13 +252,19 @@ class GpuAmg {
   // mode).  In mixed mode the CG operator reads hi/lo only, so an assembler
   // may leave a.v64 stale after the structure-defining first setup.
   bool level0_fp32_fresh = false;
+  // Such an assembler's way to write a.v64 too (and the FP32 values again).
+  std::function<void()> write_level0_fp64;
+  // reuse setups run in FP32: mixed precision, until one fails
+  bool fp32_reuse() const { return mixed() && opt.reuse && !fp64_reuse_; }
   MfOp mf;
   // Level 0: the caller fills levels[0]->a (device CSR with FP64 values, and
   // FP32 values in mixed mode), its node layout (first) and pattern (apat),
   // and the near-null space.
   Level& level0();
   // structure_changed: rebuild aggregates / patterns (first setup or a new
-  // structure); otherwise reuse them when opt.reuse.
+  // structure); otherwise reuse them when opt.reuse.  An FP32 reuse setup whose
+  // operators lose their definiteness to rounding is done again in FP64, as
+  // are the structure's later ones.
   void setup(bool structure_changed);
   bool ready() const { return ready_; }
   // level-0 FP32 hi/lo values from the FP64 ones (mixed mode)
@@ -321,6 +328,7 @@ class GpuAmg {
 
  private:
   bool ready_ = false;
+  bool fp64_reuse_ = false;  // FP32 was too short for a reuse setup of this structure
   i32 nc_ = 0;
   DBuf<double> lz_ab_;        // Lanczos coefficients and scalars of the level in setup
   PinnedBuf<double> lz_host_;
@@ -330,7 +338,8 @@ class GpuAmg {
   SolveWork main_;
   std::vector<std::unique_ptr<SolveWork>> extra_;
 
-  void numeric_level(size_t l);
+  void setup_once(bool reuse, bool fp32);
+  void numeric_level(size_t l, bool fp32);
   template <class T>
   void lanczos(size_t l, int m, double* ab);
   void build_transfer(size_t l);

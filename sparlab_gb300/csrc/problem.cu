@@ -291,6 +291,7 @@ void GpuProblem::build() {
     amg.mf.scale2 = sf2.p;
   }
   amg.mf.scale64 = sf.p;  // the FP64 SIMP factors (matrix-free CG operator)
+  amg.write_level0_fp64 = [this] { assemble(sf.p, sf2.p, false); };
   df.alloc(ne_s);
   dc_dphys.alloc(ne_s);
   dc_dx.alloc(ne_s);
@@ -497,8 +498,8 @@ void GpuProblem::assemble(const double* scale, const float2* scale2, bool exact)
   if (!amg.par_cg()) l0.a.v2.alloc(static_cast<size_t>(l0.a.nnz));
   if (exact) {
     launch(k_assemble_tiles<true, false>, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
-  } else if (!amg.opt.reuse) {
-    // every setup rebuilds the hierarchy from FP64 values
+  } else if (!amg.fp32_reuse()) {
+    // every setup takes FP64 values
     launch(k_assemble_tiles<false, false>, l0.a.v64.p, l0.a.v32.p, l0.a.v2.p);
   } else {
     launch(k_assemble_tiles<false, true>, nullptr, l0.a.v32.p, l0.a.v2.p);

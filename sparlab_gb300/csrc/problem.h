@@ -99,7 +99,7 @@ class GpuProblem {
   // exact: rounded products and sums in element order (the structure-
   // defining first assembly); otherwise fused multiply-adds.  scale2: the same
   // factors as (hi, lo) pairs, read by the mixed-precision reuse assembly
-  // alone (inexact, opt.reuse)
+  // alone (inexact, amg.fp32_reuse())
   void assemble(const double* scale_device, const float2* scale2_device, bool exact);
   // FP64 sum_e s_e E over level 0's pattern for a device element matrix E
   // (K_e^0, or M_e^0 for the mass), with the same kernel and order; FP32
