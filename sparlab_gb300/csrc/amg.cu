@@ -68,7 +68,7 @@ namespace {
 template <class TA, class F>
 void with_shape(const NbOp& op, F&& f) {
   if constexpr (std::is_same<TA, float>::value) {
-    // the coarse levels' 3-D operators and long restrictions: a warp a node
+    // the coarse levels' 3-D operators: a warp a node
     if (op.six) {
       f(std::integral_constant<int, kNodeWarp>{}, std::integral_constant<int, 6>{});
       return;
@@ -231,14 +231,12 @@ void convert(const A* a, B* b, i64 n, cudaStream_t s) {
 
 MfView mf_view(const MfOp& o) {
   MfView v;
-  v.dim = o.dim;
   v.nx = o.nx;
   v.ny = o.ny;
   v.nz = o.nz;
   v.nnx = o.nnx;
   v.nny = o.nny;
   v.nindex = o.nindex;
-  v.ke = o.ke;
   v.scale = o.scale;
   return v;
 }
@@ -504,11 +502,11 @@ void GpuAmg::init_reductions(SolveWork& w) {
   *w.post.p = PcgPost{};
 }
 
+thread_local int t_chain_off = 0;
+
 // Polls the post: a copy and a synchronisation of the stream cost several
 // microseconds an iteration.  The stream's state is looked at now and then,
 // so a failed launch ends the wait.
-thread_local int t_chain_off = 0;
-
 void wait_for_post(const volatile unsigned* seq, unsigned value, cudaStream_t stream) {
   for (unsigned spin = 1; *seq != value; ++spin) {
     if (spin % 64 == 0) std::this_thread::yield();

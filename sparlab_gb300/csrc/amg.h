@@ -132,8 +132,6 @@ struct Level {
   double lz_norm = 0.0;
 };
 
-// Matrix-free level-0 operator of a structured grid (see mfree.cuh), used
-// by the FP32 V-cycle and the mixed-precision CG operator when enabled.
 // Grid nodes from which the double-float CG operator and the FP32 cycle run in
 // the parity basis.  Below them the march along z is too short to hide its
 // steps' latency and K_ff's pairs sit in L2: the CG product takes 10.4 us
@@ -144,12 +142,13 @@ struct Level {
 constexpr i64 kParCgNodes = 20000;
 constexpr i64 kParCycleNodes = 150000;
 
+// Matrix-free level-0 operator of a structured grid (see mfree.cuh), used
+// by the FP32 V-cycle and the mixed-precision CG operator when enabled.
 struct MfOp {
   bool enabled = false;
   int dim = 3;
   i32 nx = 0, ny = 0, nz = 1, nnx = 0, nny = 0;
   const i32* nindex = nullptr;  // grid node -> free node or -1
-  const float* ke = nullptr;    // K_e^0, FP32
   const float* scale = nullptr; // s_e, FP32
   float ke_host[24 * 24] = {};  // K_e^0, FP32 (kernel parameter of the tiled 3-D kernel)
   // variant of the tiled 3-D kernel per mode (0..8): shape

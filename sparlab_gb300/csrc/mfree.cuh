@@ -16,11 +16,9 @@ namespace simp {
 namespace {
 
 struct MfView {
-  int dim;             // 2 or 3
   i32 nx, ny, nz;      // cells (nz = 1 in 2-D)
   i32 nnx, nny;        // nodes per axis in x, y
   const i32* nindex;   // grid node -> free node or -1
-  const float* ke;     // K_e^0 (ed x ed, row-major)
   const float* scale;  // s_e
 };
 

@@ -257,7 +257,6 @@ void GpuProblem::build() {
     for (uint8_t m : cmask_h) all_or_nothing = all_or_nothing && m == full;
     if (amg.mixed() && all_or_nothing && amg.opt.matrix_free >= 1) {
       std::vector<float> k32(d.ke.begin(), d.ke.end());
-      ke32.upload(k32);
       nindex.upload(node_index);
       MfOp& mf = amg.mf;
       mf.enabled = true;
@@ -268,7 +267,6 @@ void GpuProblem::build() {
       mf.nnx = g.nnx;
       mf.nny = g.nny;
       mf.nindex = nindex.p;
-      mf.ke = ke32.p;
       std::copy(k32.begin(), k32.end(), mf.ke_host);
       std::copy(d.ke.begin(), d.ke.end(), mf.ke64_host);
       mf.parity = dim == 3 && parity_blocks(d.ke.data(), mf.kpar);

@@ -124,7 +124,7 @@ class GpuProblem {
   void change_and_gray(OcStep& st, const double* candidate);
   DBuf<double> oc_g, oc_lo, oc_hi;  // OC candidate factors of the current update
   // matrix-free level-0 operator (mixed precision, fully free / clamped nodes)
-  DBuf<float> ke32, sf32;
+  DBuf<float> sf32;
   DBuf<float2> sf2;  // the stiffness factors as (hi, lo) pairs (mixed precision)
   DBuf<i32> nindex;
   void* stencil_d = nullptr;
