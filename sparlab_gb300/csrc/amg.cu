@@ -1174,7 +1174,7 @@ bool launch_rows(const char* name, void (*kernel)(i32, WarpRows, KArgs...), i32 
     if (smem > 48 * 1024) raise_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     const i64 units = static_cast<i64>(warps) * per;
     const i64 blocks =
-        std::max<i64>(1, std::min<i64>((static_cast<i64>(nodes) * parts + units - 1) / units, 152 * 64));
+        std::max<i64>(1, std::min<i64>((static_cast<i64>(nodes) * parts + units - 1) / units, kSms * 64));
     kernel<<<static_cast<unsigned>(blocks), warps * 32, smem, s>>>(nodes, w, args...);
     SIMP_CHECK_LAUNCH();
   };
@@ -1196,7 +1196,7 @@ static void galerkin_t(GpuAmg& g, Level& lv, Level& nv, bool last, cudaStream_t 
   constexpr bool kExact = std::is_same<T, double>::value;
   const int bf = uniform_block(lv.first);
   auto gather = [&](auto kernel) {
-    const i64 blocks = std::max<i64>(1, std::min<i64>((static_cast<i64>(lv.nnodes) * 32 + 255) / 256, 152 * 64));
+    const i64 blocks = std::max<i64>(1, std::min<i64>((static_cast<i64>(lv.nnodes) * 32 + 255) / 256, kSms * 64));
     kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(lv.nnodes, lv.d_agg.p, lv.a.ptr.p, A(lv.a),
                                                               lv.d_ppat.view(), lv.p.ptr.p, A(lv.p), lv.phat_ptr.p,
                                                               phat, lv.dinv64.p, omega, lv.d_pc_ptr.p, lv.d_pc.p);
@@ -1256,7 +1256,7 @@ static void galerkin_t(GpuAmg& g, Level& lv, Level& nv, bool last, cudaStream_t 
   const int b0 = uniform_block(lv.first);
   bool ap_done = false;
   if constexpr (X) {
-    if (lv.nnodes < 16 * 152)
+    if (lv.nnodes < 16 * kSms)
       ap_done = (b0 == 3 && b1 == 6)   ? ap_rows(k_ap_rows<T, X, 3, 6, H, 1>, PER, 3)
                 : (b0 == 6 && b1 == 6) ? ap_rows(k_ap_rows<T, X, 6, 6, 32, 1>, 1, 6)
                 : (b0 == 2 && b1 == 3) ? ap_rows(k_ap_rows<T, X, 2, 3, H, 1>, PER, 2)
@@ -1278,11 +1278,11 @@ static void galerkin_t(GpuAmg& g, Level& lv, Level& nv, bool last, cudaStream_t 
   }
   bool rap_done = false;
   if constexpr (X) {
-    if (nv.nnodes < 4 * 152)
+    if (nv.nnodes < 4 * kSms)
       rap_done = (b1 == 6 && b0 == 3)   ? rap_rows(k_rap_rows<T, X, 6, 3, 1>, 6)
                  : (b1 == 6 && b0 == 6) ? rap_rows(k_rap_rows<T, X, 6, 6, 1>, 6)
                                         : false;
-    if (!rap_done && nv.nnodes < 64 * 152)
+    if (!rap_done && nv.nnodes < 64 * kSms)
       rap_done = (b1 == 6 && b0 == 3)   ? rap_rows(k_rap_rows<T, X, 6, 3, 2>, 3)
                  : (b1 == 6 && b0 == 6) ? rap_rows(k_rap_rows<T, X, 6, 6, 2>, 3)
                  : (b1 == 3 && b0 == 2) ? rap_rows(k_rap_rows<T, X, 3, 2, 1>, 3)
@@ -1669,7 +1669,7 @@ void GpuAmg::pcg_tail(SolveWork& w, float2* psplit) {
     chain_launch(k_pcg_rz<TZ>, red_blocks(n), kRedThreads, 0, stream, residual(w), z, n, planes, w.part.p, w.scalars());
     SIMP_CHECK_LAUNCH();
     // four values a thread where that still gives every SM eight blocks
-    const bool four = n >= 4 * 256 * 8 * 152;
+    const bool four = n >= 4 * 256 * 8 * kSms;
     chain_launch(four ? k_pcg_direction<TZ, 4> : k_pcg_direction<TZ, 1>, (static_cast<i64>(n) + (four ? 1023 : 255)) / (four ? 1024 : 256),
                  256, 0, stream, w.pp.p, z, n, planes, w.scalars(), psplit, mf_cg() ? w.p32.p : nullptr);
     SIMP_CHECK_LAUNCH();

@@ -50,6 +50,10 @@ extern thread_local int64_t t_launches;
     SIMP_CUDA(cudaGetLastError());      \
   } while (0)
 
+// SMs of a GB300, where a rule that was measured on one counts blocks, nodes or
+// CTAs for each of them.
+constexpr int kSms = 152;
+
 // Launch of a kernel whose first statement is chain_start() (kernels.cuh): it
 // may be scheduled while the stream's previous kernel drains, and waits there,
 // before its first access, until that kernel has completed.  The CG iteration,

@@ -137,7 +137,7 @@ __device__ __forceinline__ double block_sum(double v) {
 // blocks would fill the slots that happen to be free and the SMs would have
 // unequal shares of it (46800 rows, FP64, 731 blocks after 731: a CG iteration
 // of 227 us against 181 without any overlap).
-constexpr unsigned kChainBlocks = 304;
+constexpr unsigned kChainBlocks = 2 * kSms;
 __device__ __forceinline__ bool chain_start() {
   unsigned lane;
   asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%laneid;" : "=r"(lane)::"memory");

@@ -276,7 +276,7 @@ static bool wgrad_on_tensor_cores(const WgradSpec& s) {
          s.cout <= s.cdy && aligned(s.dy);
 }
 
-constexpr int kWgWalkers = 152;  // CTAs over all groups: one per SM
+constexpr int kWgWalkers = kSms;  // CTAs over all groups: one per SM
 
 static void wgrad_tc_launch(const WgradSpec& s, float* part, cudaStream_t stream) {
   wg::Args a{};
