@@ -887,7 +887,7 @@ void GpuAmg::lanczos(size_t l, int m, double* ab) {
   if (mixed()) lv.dinv32.alloc(n);
   k_level_start<T><<<grid_for(n, 256), 256, 0, stream>>>(n, lv.d_node_of.p, lv.d_first.p, lv.d_self.p,
                                                          lv.d_apat.view(), lv.a.ptr.p, values, lv.lz_start.p,
-                                                         lv.lz_norm, lv.dinv64.p, lv.dinv32.p, s, w, t, v, planes, sc);
+                                                         lv.dinv64.p, lv.dinv32.p, s, w, t, v, planes, sc);
   SIMP_CHECK_LAUNCH();
   if constexpr (f32)
     if (matrix_free) lz_y_.alloc(static_cast<size_t>(n));
@@ -919,15 +919,17 @@ void GpuAmg::numeric_level(size_t l, bool fp32) {
   const i32 n = lv.n;
   make_ops(l);
   lv.dinv64.alloc(n);
-  // Lanczos on D^-1/2 A D^-1/2 with the reference's start vector (its norm
-  // made once per size); the scalars stay in device memory: the steps after a
+  // Lanczos on D^-1/2 A D^-1/2 with the reference's start vector (made once
+  // per size); the scalars stay in device memory: the steps after a
   // breakdown change nothing, and the host reads all coefficients and the
   // diagonal's status once (a bad diagonal only makes them garbage)
   if (lv.lz_start.n != static_cast<size_t>(n)) {
     std::vector<double> h(static_cast<size_t>(n));
     for (i32 i = 0; i < n; ++i) h[i] = 1.0 + 0.5 * std::sin(1.7 * static_cast<double>(i) + 0.3);
     lv.lz_start.upload(h, stream);
-    lv.lz_norm = std::sqrt(dot(lv.lz_start.p, lv.lz_start.p, n));
+    const double norm = std::sqrt(dot(lv.lz_start.p, lv.lz_start.p, n));
+    for (double& v : h) v /= norm;
+    lv.lz_start.upload(h, stream);
   }
   const int m = std::max(1, std::min<int>(opt.lanczos_steps, n));
   // alpha_j, beta_j pairs, then the scalars

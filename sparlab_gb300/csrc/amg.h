@@ -128,8 +128,7 @@ struct Level {
   double inv_theta = 0.0;
   DBuf<double> lz[4];  // Lanczos work vectors (FP64 setups)
   DBuf<float> lz32[4];  // (FP32 reuse setups)
-  DBuf<double> lz_start;  // Lanczos start vector (depends on n only) and its norm
-  double lz_norm = 0.0;
+  DBuf<double> lz_start;  // Lanczos start vector, of unit norm (depends on n only)
 };
 
 // Grid nodes from which the double-float CG operator and the FP32 cycle run in

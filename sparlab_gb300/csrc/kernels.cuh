@@ -456,8 +456,8 @@ __global__ void k_add_to(i64 n, const TX* __restrict__ d, TX* __restrict__ x) {
 // product and k_lz_post), then k_lz_norm; the last block of each adds the
 // partials in order.  The vector of a step stays unnormalised: u = beta_{j-1}
 // v_j is in w and t = s u is the operator's input, scaled in the rows'
-// epilogue, so no pass divides by beta (the first one is the start vector over
-// its norm, divided in FP64, with beta_0 = 1).  FP32 vectors (the
+// epilogue, so no pass divides by beta (the first one is the start vector, of unit
+// norm, with beta_0 = 1).  FP32 vectors (the
 // mixed-precision reuse setups) take FP32 arithmetic with FP64 scalars, and a
 // row's products are added up in FP64: GB300 runs FP64 at 1/64 of the FP32
 // rate, so a block of rows leaves its products in shared memory and one warp
@@ -572,13 +572,13 @@ __global__ void k_lz_reset(LzScalars* sc) {
 }
 
 // Inverse diagonal of a level (1 / a_ii; the first entry that is not positive
-// is recorded) and the Lanczos start: s = sqrt(1 / a_ii), w = start / norm,
-// t = s w, v = 0.  planes > 0: dinv32, s, w, t and v in component planes of that many
+// is recorded) and the Lanczos start: s = sqrt(1 / a_ii), w = start, t = s w,
+// v = 0.  planes > 0: dinv32, s, w, t and v in component planes of that many
 // nodes (three unknowns a node).
 template <class T>
 __global__ void k_level_start(i32 n, const i32* __restrict__ node_of, const i32* __restrict__ first,
                               const i32* __restrict__ self_slot, NodeView a, const i32* __restrict__ rowptr,
-                              const T* __restrict__ val, const double* __restrict__ start, double norm, double* __restrict__ dinv,
+                              const T* __restrict__ val, const double* __restrict__ start, double* __restrict__ dinv,
                               float* __restrict__ dinv32, T* __restrict__ s, T* __restrict__ w, T* __restrict__ t,
                               T* __restrict__ v, i64 planes, LzScalars* __restrict__ sc) {
   for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
@@ -591,7 +591,7 @@ __global__ void k_level_start(i32 n, const i32* __restrict__ node_of, const i32*
     dinv[i] = inv;
     const i64 o = planes > 0 ? (i % 3) * planes + i / 3 : i;
     if (dinv32) dinv32[o] = static_cast<float>(inv);
-    const T si = static_cast<T>(sqrt(inv)), wi = static_cast<T>(start[i] / norm);
+    const T si = static_cast<T>(sqrt(inv)), wi = static_cast<T>(start[i]);
     s[o] = si;
     w[o] = wi;
     t[o] = si * wi;
