@@ -241,7 +241,10 @@ struct ParIo<ParDf> {
 };
 
 // Two resident blocks bound the registers (FP32, 10 warps: 96; double-float, 6
-// warps: 168); three spill (192x96x96: double-float 422 against 319 us).
+// warps: 168); three spill (192x96x96: double-float 422 against 319 us).  They
+// are full, so nothing that a layer can form again is kept across layers: with
+// the coefficients and the sizes of node and cell planes kept, modes 3 and 5
+// spill 8 bytes (192x96x96 design pass 62.4 against 61.0 ms).
 template <int MODE, class AR, int TY>
 __global__ void __launch_bounds__(32 * (TY + 2), 2) k_mf3_par(MfView m, typename ParIo<AR>::Args a,
                                                             const __grid_constant__ typename AR::Ke ke, int chunk) {
@@ -264,18 +267,14 @@ __global__ void __launch_bounds__(32 * (TY + 2), 2) k_mf3_par(MfView m, typename
   const bool edge_in = row_in && lane == 31 && gx + 1 < m.nnx;  // the right neighbour of lane 31
   const bool cell_in = gx >= 0 && gx < m.nx && gy >= 0 && gy < m.ny;
   const bool owns = node_in && lane >= 1 && j >= 1 && j <= TY;
-  // (32-bit indices: the unknowns are counted in 32 bits)
-  const i32 plane = m.nnx * m.nny, node0 = gy * m.nnx + gx;
-  const i32 cplane = m.nx * m.ny, cell0 = gy * m.nx + gx;
-  float c0 = 0.0f, c1 = 0.0f;
-  Io::template coefs<MODE>(a, c0, c1);
 
   // free-node index of this thread's column (and lane 31's neighbour) in layer L
+  // (32-bit indices: the unknowns are counted in 32 bits)
   auto index_of = [&](i32 L, i32& I, i32& E) {
     I = E = -1;
     if (L >= 0 && L < nnz) {
-      if (node_in) I = m.nindex[L * plane + node0];
-      if (edge_in) E = m.nindex[L * plane + node0 + 1];
+      if (node_in) I = m.nindex[(L * m.nny + gy) * m.nnx + gx];
+      if (edge_in) E = m.nindex[(L * m.nny + gy) * m.nnx + gx + 1];
     }
   };
   auto values_of = [&](i32 I, Raw (&u)[3]) {
@@ -322,7 +321,7 @@ __global__ void __launch_bounds__(32 * (TY + 2), 2) k_mf3_par(MfView m, typename
       }
     }
     const V sc = Io::value(sn);  // scale of cell layer L - 1
-    if (L < z1) sn = cell_in && L >= 0 && L < m.nz ? Io::scale(m, a, L * cplane + cell0) : Raw{};
+    if (L < z1) sn = cell_in && L >= 0 && L < m.nz ? Io::scale(m, a, (L * m.ny + gy) * m.nx + gx) : Raw{};
     const bool out = owns && L - 2 >= z0 && Ib >= 0;
     typename Io::In in;
     if (out) Io::template fetch<MODE>(a, Ib, in);
@@ -337,7 +336,11 @@ __global__ void __launch_bounds__(32 * (TY + 2), 2) k_mf3_par(MfView m, typename
           const V as = AR::add(hs, low[0][k]), ad = AR::add(hd, low[1][k]);
           o[k] = AR::add(AR::up(AR::add(as, ad)), AR::sub(as, ad));
         }
-        if (out) Io::template store<MODE>(a, Ib, o, in, c0, c1);
+        if (out) {
+          float c0 = 0.0f, c1 = 0.0f;
+          Io::template coefs<MODE>(a, c0, c1);
+          Io::template store<MODE>(a, Ib, o, in, c0, c1);
+        }
       }
       if (L <= z1) {
         // xy modes of layer L: bit 0 difference along x, bit 1 along y
