@@ -684,13 +684,14 @@ def run_own(args):
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / (kms * 1e-3) / 1e9
     if args.precision == "fp64":
-        operator = f"k_rows_apply<4,{spec.dim},0,double> (level-0 K_ff operator of the CG, FP64 values; FP64-pipe bound on GB300)"
+        operator, bound = (f"k_rows_apply<4,{spec.dim},0,double> (level-0 K_ff operator of the CG, FP64 values)",
+                           "fp64 pipe")
     elif alg_bytes < 8.0 * nnz:  # no stored values among its bytes
-        operator = ("k_mf3_par<0,ParDf> (level-0 operator of the CG, matrix-free in the parity basis, double-float "
-                    "arithmetic on the FP32 pipes; bound by their issue rate)")
+        operator, bound = ("k_mf3_par<0,ParDf> (level-0 operator of the CG, matrix-free in the parity basis, "
+                           "double-float arithmetic on the FP32 pipes)", "instruction issue")
     else:
-        operator = (f"k_rows_apply_df<4,{spec.dim},0> (level-0 K_ff operator of the CG, double-float values and "
-                    "arithmetic on the FP32 pipes)")
+        operator, bound = (f"k_rows_apply_df<4,{spec.dim},0> (level-0 K_ff operator of the CG, double-float values "
+                           "and arithmetic on the FP32 pipes)", "hbm")
     traffic = None
     prof = os.path.join(ROOT, "profiles", "spmv_traffic.json")
     if os.path.exists(prof):
@@ -789,7 +790,7 @@ def run_own(args):
                              for k, v in _lib.autotune_report().items()},
                 "plain_fp64": plain,
                 "oracle_check": oracle_check},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"bound": bound, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic,
                      "kernel": operator,
                      "bytes_per_launch": alg_bytes, "ms_per_launch": kms,
