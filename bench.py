@@ -692,6 +692,7 @@ def run_own(args):
     else:
         operator, bound = (f"k_rows_apply_df<4,{spec.dim},0> (level-0 K_ff operator of the CG, double-float values "
                            "and arithmetic on the FP32 pipes)", "hbm")
+    kff_bytes = nnz * {"fp64 pipe": 8, "instruction issue": 4, "hbm": 12}[bound]  # what a step reads of it
     traffic = None
     prof = os.path.join(ROOT, "profiles", "spmv_traffic.json")
     if os.path.exists(prof):
@@ -771,10 +772,10 @@ def run_own(args):
                 "level0_tensor_cores": int(prob.options.tensor_cores),
                 "load_case_solves": ("one graph, fused multi-RHS CG operator" if together == "graph" else
                                      "concurrent" if together else "sequential"),
-                "l2": ("working set (K_ff %.2f GB) larger than the 129 MB L2" % (nnz * 12 / 1e9)
-                       if nnz * 12 > 129e6 else
+                "l2": ("working set (K_ff %.2f GB) larger than the 129 MB L2" % (kff_bytes / 1e9)
+                       if kff_bytes > 129e6 else
                        "working set (K_ff %.3f GB) fits in the 129 MB L2; not flushed between steps"
-                       % (nnz * 12 / 1e9)),
+                       % (kff_bytes / 1e9)),
                 "amg_levels": st["num_levels"],
                 "operator_complexity": round(st["operator_complexity"], 6),
                 "cg_iterations_per_step": [r.linear_iterations for r in recs],

@@ -42,7 +42,8 @@ extern "C" {
 #define SIMP_CUDA_ERROR 6
 
 /* FP64: every operator, vector and scalar in FP64.  MIXED: the V-cycle and
- * the reuse setups in FP32 (level 0 matrix-free on structured grids), the CG
+ * the reuse setups in FP32 (level 0 matrix-free on structured grids; a setup
+ * whose coarse operators FP32 leaves indefinite is done in FP64), the CG
  * operator in double-float arithmetic (K_ff as float pairs, ~2^-44 relative
  * to FP64); CG vectors and scalars, the true-residual restarts and the
  * coarsest dense inverse are FP64 in both. */

@@ -7,7 +7,8 @@
 // arithmetic).  SIMP_PRECISION_MIXED keeps FP32 copies of every operator,
 // prolongator and restriction and runs the V-cycle (smoother, residuals,
 // transfers; level 0 matrix-free on structured grids), the Lanczos estimates
-// and the reused-structure Galerkin products in FP32.  CG itself -- its
+// and the reused-structure Galerkin products in FP32 (in FP64 for structures
+// where FP32 leaves a coarse operator indefinite).  CG itself -- its
 // operator, vectors, scalars and the true-residual restarts -- and the
 // coarsest dense inverse stay FP64 in both modes, so both stop on the same
 // FP64 residual test.

@@ -29,12 +29,14 @@
 // or double-float (the CG operator: (hi, lo) float pairs in, FP64 output and
 // right-hand side).
 //
-// Bound by instruction issue (FP32 at 120x64x64: 56 % of the issue slots, 0.2
-// of the load/store wavefronts, the rest barrier and load latency at 18 warps
-// an SM).  Measured, us a launch, before -> after: y = A x double-float 700
-// -> 195 at 192x96x96 (the assembled rows read 3.8 GB, this 0.1 GB) and 97 ->
-// 39 at 96x48x48; FP32 Chebyshev step 87 -> 68 and 16.9 -> 14.8, the other
-// modes 79-86 -> 43-54 and 15-16.9 -> 12.8.  Errors against FP64 fall too:
+// Bound by instruction issue: 965 instructions a node, most of them node
+// indices and their tests, addresses, shuffles and exchanges beside the
+// arithmetic (FP32 at 120x64x64: 56 % of the issue slots, 0.2 of the load/store
+// wavefronts, the rest barrier and load latency at 18 warps an SM).  Measured,
+// us a launch, before -> after: y = A x double-float 700 -> 193 at 192x96x96
+// (the assembled rows read 3.8 GB, this 0.1 GB) and 97 -> 39 at 96x48x48; FP32
+// Chebyshev step 87 -> 60 and 16.9 -> 14.8, the other modes 79-86 -> 43-52 and
+// 15-16.9 -> 12.8.  Errors against FP64 fall too:
 // double-float 8.6e-15 -> 3.6e-15 (2-norm, random x) and 1.7e-12 -> 3.3e-13
 // (smooth x), FP32 7.2e-8 -> 6.8e-8 and 1.1e-5 -> 8.5e-6.
 #pragma once

@@ -15,7 +15,8 @@ from sparlab_gb300.topopt import GpuSimpProblem
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,solid", [((140, 4, 4), True), ((260, 4, 4), False), ((300, 8, 8), True), ((460, 8, 8), True)])
+@pytest.mark.parametrize("n,solid", [((140, 4, 4), True), ((260, 4, 4), False), ((300, 8, 8), True), ((460, 8, 8), True),
+                                     ((700, 15, 15), True)])  # level-0 vectors in planes
 def test_evaluations_after_the_first(n, solid):
     spec = P.hex8_cantilever(*n, 0.3, "slender")
     spec.warm_start = 0
