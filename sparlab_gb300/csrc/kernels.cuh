@@ -456,12 +456,12 @@ __global__ void k_add_to(i64 n, const TX* __restrict__ d, TX* __restrict__ x) {
 // product and k_lz_post), then k_lz_norm; the last block of each adds the
 // partials in order.  The vector of a step stays unnormalised: u = beta_{j-1}
 // v_j is in w and t = s u is the operator's input, scaled in the rows'
-// epilogue, so no pass divides by beta (the first one is the start vector, of unit
-// norm, with beta_0 = 1).  FP32 vectors (the
-// mixed-precision reuse setups) take FP32 arithmetic with FP64 scalars, and a
-// row's products are added up in FP64: GB300 runs FP64 at 1/64 of the FP32
-// rate, so a block of rows leaves its products in shared memory and one warp
-// adds them, 7 FP64 additions a block where sums in every warp take 32.
+// epilogue, so no pass divides by beta (the first u is the start vector, of
+// unit norm, with beta_0 = 1).  FP32 vectors (the mixed-precision reuse setups)
+// take FP32 arithmetic with FP64 scalars, and a row's products are added up in
+// FP64: GB300 runs FP64 at 1/64 of the FP32 rate, so a block of rows leaves its
+// products in shared memory and one warp adds them, 7 FP64 additions a block
+// where sums in every warp take 32.
 // ---------------------------------------------------------------------------
 // Device scalars of a level's Lanczos run (alpha_j and beta_j follow the host's
 // order in an array of their own).
